@@ -433,14 +433,15 @@ int init_impl(const islbm_params *pp, islbm_handle *h) {
     h->steps = 0;
     h->use_tiled = false;
     h->paired = false;
+    h->chunked = false;
+    int sms = 0;
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+    double wx0[7], wx2[7], wy0[7], wy2[7];
+    for (int a = 0; a < 7; a++) {   // uniform spacing: the weights of the first node serve all
+        wx0[a] = h->g.XP0[(size_t)a*h->g.NX6 + 3]; wx2[a] = h->g.XP2[(size_t)a*h->g.NX6 + 3];
+        wy0[a] = h->g.YP0[(size_t)a*h->g.NYD6 + 3]; wy2[a] = h->g.YP2[(size_t)a*h->g.NYD6 + 3];
+    }
     if (p.kernel == ISLBM_KERNEL_TILED || p.kernel == ISLBM_KERNEL_AUTO || p.kernel == ISLBM_KERNEL_TILED_SINGLE) {
-        int sms = 0;
-        CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
-        double wx0[7], wx2[7], wy0[7], wy2[7];
-        for (int a = 0; a < 7; a++) {   // uniform spacing: the weights of the first node serve all
-            wx0[a] = h->g.XP0[(size_t)a*h->g.NX6 + 3]; wx2[a] = h->g.XP2[(size_t)a*h->g.NX6 + 3];
-            wy0[a] = h->g.YP0[(size_t)a*h->g.NYD6 + 3]; wy2[a] = h->g.YP2[(size_t)a*h->g.NYD6 + 3];
-        }
         // the paired-node kernel where the grid allows it, else the one-node-per-thread kernel
         if (p.kernel != ISLBM_KERNEL_TILED_SINGLE && pair_supported(k, p.precision) &&
             make_pair_const(k, p.precision, wx0, wx2, wy0, wy2, sms, &h->tiled) == 0) {
@@ -452,6 +453,10 @@ int init_impl(const islbm_params *pp, islbm_handle *h) {
             h->use_tiled = true;
         }
         if (p.kernel != ISLBM_KERNEL_AUTO && !h->use_tiled) { g_last = "tiled kernel does not support this grid"; return ISLBM_ERR_NOT_SUPPORTED; }
+    }
+    if (p.kernel == ISLBM_KERNEL_AUTO && !h->use_tiled) {
+        CK(make_chunk_const(k, p.precision, p.les_cs > 0.0, wx0, wx2, wy0, wy2, sms, &h->chunk));
+        h->chunked = true;
     }
     CK(cudaStreamSynchronize(h->stream));
     return ISLBM_OK;
@@ -520,6 +525,7 @@ int islbm_step(islbm_handle *h, int nsteps) {
     L.les = h->p.les_cs > 0.0;
     L.stream = h->stream;
     L.tiled = &h->tiled;
+    L.chunk = &h->chunk;
     for (int s = 0; s < nsteps; s++) {
         const unsigned long long n = h->steps + 1;
         L.fo = h->fbuf[h->cur];
@@ -529,7 +535,7 @@ int islbm_step(islbm_handle *h, int nsteps) {
         L.mass = h->p.mass_interval > 0 && (n % (unsigned long long)h->p.mass_interval) == 0ULL;
         L.macros_on = (s == nsteps - 1);
         for (int m = 0; m < 4; m++) L.macros[m] = h->macros[m];
-        cudaError_t e = h->paired ? launch_step_pair(L) : h->use_tiled ? launch_step_tiled(L) : launch_step_gather(L);
+        cudaError_t e = h->paired ? launch_step_pair(L) : h->use_tiled ? launch_step_tiled(L) : h->chunked ? launch_step_chunk(L) : launch_step_gather(L);
         if (e != cudaSuccess) return cuda_fail(e, "step kernel launch");
         h->cur = 1 - h->cur;
         h->steps = n;

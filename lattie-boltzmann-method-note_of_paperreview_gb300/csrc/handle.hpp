@@ -7,6 +7,7 @@
 #include "geometry.hpp"
 #include "step_launch.hpp"
 #include "step_tiled.hpp"
+#include "step_chunk.hpp"
 
 using namespace islbm;
 
@@ -38,6 +39,8 @@ struct islbm_handle {
 
     double *xfer = nullptr;    // FP64 transfer buffer of N values for host copies (first use)
     TiledConst tiled{};
+    bool chunked = false;      // the chunk-marching kernel (step_chunk.cu) steps this solve
+    ChunkConst chunk{};
     PairMaps pmaps{};          // tensor maps of fbuf[0], fbuf[1] for the paired kernel's copies
 };
 

@@ -56,7 +56,7 @@ __device__ __forceinline__ V2 &operator-=(V2 &a, V2M m) { a = vfma(vneg(m.a), m.
 __device__ __forceinline__ V2 vrcp(V2 a) { return V2(__fdividef(1.f, a.v.x), __fdividef(1.f, a.v.y)); }
 __device__ __forceinline__ float sqrt_nn(float v) { return v > 0.f ? v*rsqrtf(v) : 0.f; }
 
-// Collision tail of C/evolution.h:597-652 for a node pair, the operator of collide_node_pairs
+// Collision tail of C/evolution.h:597-652 for a node pair, the operator of collide_pairs
 // (step_common.cuh) on packed pairs: mass correction, density and velocity from the opposite-
 // direction pair sums and differences, their non-equilibrium parts, the Smagorinsky rate from
 // Q = Pi:Pi (LES), the generated sparse MRT relaxation and the body force.

@@ -1,0 +1,451 @@
+// Chunk-marching step kernel: the separable interpolation on any grid and storage format.
+//
+// Same step as stream_collide (C/evolution.h:358-684). It serves FP64 (the parity precision) and
+// every grid without a tiled layout (spanwise widths other than the tiled ones, streamwise counts
+// that are no multiple of a tile's rows), where the gather kernel evaluates each departure point's
+// 7 x 7 x 7 stencil by itself: about 2,500 multiply-adds and adds per node. Here the streamwise and
+// spanwise filters are applied once per plane and node and the xi combination once per target,
+// 252 multiply-adds per node, as the tiled kernels do:
+//   * a CTA of 128 threads owns a tile of W x H <= 32 columns (one lane each) and marches upward
+//     through a wall-normal segment in chunks of CHUNK planes;
+//   * phase A filters 7, 8, 9, 10 in y on the chunk's new planes, for the tile's columns and
+//     three halo columns on each side, into shared memory; phase B filters them in x, the other
+//     populations in y or x straight from global memory (L1 / L2), and stores the 16 values of
+//     every column in a ring of CHUNK + 6 planes in shared memory; phase C combines seven planes
+//     per target along xi, collides and stores. The four warps take different planes (A, B)
+//     and targets (C) of a chunk, so a chunk costs two CTA barriers and no other synchronisation;
+//   * bounce-back (BFL) rows: the 7 x 7 (y, xi) sums of the flagged rows are spread over the whole
+//     CTA before phase C, with the halo columns, so that only a 7-tap x filter is left per node.
+//     The gather kernel's per-thread 343-point sums were the critical path on small grids.
+//
+// Bound: in FP64 the FP64 pipe (GB300 issues 2 FP64 lanes per clock and SM: about 560 operations per
+// node take 5.8 ms on 256x128x192); in FP32 the load/store and issue rate. Measured against the
+// gather kernel, per step: FP64 256x128x192 (LES) 28.2 -> 6.97 ms, FP64 64x32x48 506 -> 135 us, FP32
+// 187x91x131 (LES) 2,956 -> 232 us (9.6 GLUPS).
+#include <algorithm>
+#include <cstring>
+
+#include "step_common.cuh"
+#include "step_launch.hpp"
+#include "step_chunk.hpp"
+
+namespace islbm {
+
+namespace {
+
+constexpr int NT = 128, P = 32, GROUPS = NT/P;
+constexpr int CHUNK = 8, RING = CHUNK + 6;
+
+// four values of one node (FP32: one 16-byte access, FP64: two)
+template <class C> struct alignas(16) Quad { C a, b, c, d; };
+
+template <class C> __host__ __device__ constexpr size_t ring_bytes() { return (size_t)RING*4*P*sizeof(Quad<C>); }
+
+__device__ __forceinline__ int wrap_near(int v, int n) {   // v in [-n, 2n)
+    return v < 0 ? v + n : (v >= n ? v - n : v);
+}
+__device__ __forceinline__ int wrap_any(int v, int n) {
+    v %= n;
+    return v < 0 ? v + n : v;
+}
+
+template <class S, bool LES>
+struct Chunk {
+    using C = typename Storage<S>::C;
+    const S *__restrict__ fo;
+    S *__restrict__ fn;
+    Tables<C> T;
+    StepConst k;
+    ChunkConst cc;
+    Ctrl *ctrl;
+    unsigned long long n;
+    C *rho_out, *u_out, *v_out, *w_out;
+    C ux0[7], ux2[7], uy0[7], uy2[7];   // FP32: uniform spacing, the weights of the first node
+    int macros_on, mass_on;
+
+    __device__ __forceinline__ C val(const S *p) const { return to_c(__ldg(p)); }   // stored value (a deviation for FP16 / BF16)
+    __device__ __forceinline__ C full(const S *p, C r) const { if constexpr (Storage<S>::dev) return val(p) + r; else return val(p); }
+    __device__ __forceinline__ static C ref(int q) { return Storage<S>::dev ? (C)dev_ref(q) : C(0); }
+
+    // Lagrange weights. FP64 takes each node's own: they differ from the first node's by the rounding
+    // of the node positions (about 1e-14), which the 1e-12 parity over a thousand steps would see
+    __device__ __forceinline__ C wx0(int a, int x) const { if constexpr (sizeof(C) == 8) return __ldg(T.wx0 + (size_t)a*k.NX + x); else return ux0[a]; }
+    __device__ __forceinline__ C wx2(int a, int x) const { if constexpr (sizeof(C) == 8) return __ldg(T.wx2 + (size_t)a*k.NX + x); else return ux2[a]; }
+    __device__ __forceinline__ C wy0(int b, int y) const { if constexpr (sizeof(C) == 8) return __ldg(T.wy0 + (size_t)b*k.NY + y); else return uy0[b]; }
+    __device__ __forceinline__ C wy2(int b, int y) const { if constexpr (sizeof(C) == 8) return __ldg(T.wy2 + (size_t)b*k.NY + y); else return uy2[b]; }
+
+    __device__ __forceinline__ int base(int t) const { return min(max(t - 3, 0), k.NZ - 7); }
+
+    // phase A: y filter of 7, 8, 9, 10 on planes p0 .. p0 + np - 1, columns x0 - 3 .. x0 + W + 2
+    __device__ __forceinline__ void halo_quads(Quad<C> *qb, int p0, int np, int x0, int y0) const {
+        const int WH = cc.W + 6, HW = cc.H*WH, NX = k.NX, NY = k.NY;
+        const size_t N = (size_t)NX*NY*k.NZ;
+        for (int i = threadIdx.x; i < np*HW; i += NT) {
+            const int pl = i/HW, r = i - pl*HW, yl = r/WH, xx = r - yl*WH;
+            const int y = y0 + yl;
+            if (y >= NY) continue;
+            const S *b = fo + (size_t)(p0 + pl)*NY*NX + wrap_any(x0 + xx - 3, NX);
+            C s7 = 0, s8 = 0, s9 = 0, s10 = 0;
+#pragma unroll
+            for (int j = 0; j < 7; j++) {
+                const S *p = b + (size_t)wrap_near(y - 3 + j, NY)*NX;
+                const C w0 = wy0(j, y), w2 = wy2(j, y);
+                s7 += w0*val(p + 7*N);
+                s8 += w0*val(p + 8*N);
+                s9 += w2*val(p + 9*N);
+                s10 += w2*val(p + 10*N);
+            }
+            qb[i] = Quad<C>{s7, s8, s9, s10};
+        }
+    }
+
+    struct Col {
+        int x, y, xl, yl;
+        bool on;
+        int xo[7];      // wrapped x of the spanwise stencil
+        int yo[7];      // row offsets (wrapped y times NX) of the streamwise stencil
+    };
+
+    // phase B: ring values of one column on one plane; ring order 3, 4, 5, 6 | 7, 8, 9, 10 |
+    // 11, 12, 13, 14 | 15, 16, 17, 18
+    __device__ __forceinline__ void filter(const Col &L, const Quad<C> *qrow, int p, Quad<C> *slot) const {
+        const int NX = k.NX, NY = k.NY;
+        const size_t N = (size_t)NX*NY*k.NZ;
+        const S *pl = fo + (size_t)p*NY*NX;
+        {
+            const S *b = pl + L.x;
+            Quad<C> g{0, 0, 0, 0}, h{0, 0, 0, 0};
+#pragma unroll
+            for (int j = 0; j < 7; j++) {
+                const S *r = b + L.yo[j];
+                const C w0 = wy0(j, L.y), w2 = wy2(j, L.y);
+                g.a += w0*val(r + 3*N);
+                g.b += w2*val(r + 4*N);
+                h.a += w0*val(r + 15*N);
+                h.b += w2*val(r + 16*N);
+                h.c += w0*val(r + 17*N);
+                h.d += w2*val(r + 18*N);
+            }
+            g.c = val(b + L.yo[3] + 5*N);
+            g.d = val(b + L.yo[3] + 6*N);
+            slot[0*P] = g;
+            slot[3*P] = h;
+        }
+        {
+            const S *b = pl + L.yo[3];
+            Quad<C> g{0, 0, 0, 0}, h{0, 0, 0, 0};
+#pragma unroll
+            for (int a = 0; a < 7; a++) {
+                const S *r = b + L.xo[a];
+                const C w0 = wx0(a, L.x), w2 = wx2(a, L.x);
+                h.a += w0*val(r + 11*N);
+                h.b += w2*val(r + 12*N);
+                h.c += w0*val(r + 13*N);
+                h.d += w2*val(r + 14*N);
+                const Quad<C> v = qrow[a];
+                g.a += w0*v.a;
+                g.b += w2*v.b;
+                g.c += w0*v.c;
+                g.d += w2*v.d;
+            }
+            slot[1*P] = g;
+            slot[2*P] = h;
+        }
+    }
+
+    // BFL rows: which sums a flagged row needs. Kinds 0..3 (with the halo columns): 7, 8, 9, 10 from
+    // their opposites; kinds 4..7: 3, 4, 15, 16. The flag type of a kind and its source population
+    // and weight sets (C/evolution.h:505-572).
+    __device__ __forceinline__ static int kind_flag(int kd) { return kd < 2 ? 0 : kd < 4 ? 1 : kd - 4; }
+    __device__ __forceinline__ static int kind_src(int kd) { return kd < 4 ? 10 - kd : kd == 4 ? 4 : kd == 5 ? 3 : kd == 6 ? 18 : 17; }
+    __device__ __forceinline__ static int kind_yset(int fl) { return fl == 0 ? B_YB378 : fl == 1 ? B_YB4910 : fl == 2 ? B_YB15 : B_YB16; }
+    __device__ __forceinline__ static int kind_zset(int fl) { return fl == 0 ? B_XIB378 : fl == 1 ? B_XIB4910 : fl == 2 ? B_XIB15 : B_XIB16; }
+
+    __device__ __forceinline__ C bw(int s, int a, int idx) const {
+        const int nb = 2*k.NYD6;
+        return idx < nb ? __ldg(T.bfl_w + ((size_t)s*7 + a)*nb + idx) : C(0);
+    }
+
+    // (y, xi) sums of the flagged rows z = z0 .. z1 - 1 of the tile:
+    // bf[((z*H + yl)*8 + kind)*(W + 6) + xx]. The flagged (row, kind) pairs are listed first, so that
+    // all of them are summed in one pass of the CTA (row after row, their load latencies add up).
+    __device__ __forceinline__ void bfl_sums(C *bf, int z0, int z1, int x0, int y0) const {
+        __shared__ int count;
+        __shared__ unsigned short list[2*P*8];
+        const int WH = cc.W + 6, NX = k.NX, NY = k.NY, nb = 2*k.NYD6;
+        const size_t N = (size_t)NX*NY*k.NZ;
+        if (threadIdx.x == 0) count = 0;
+        __syncthreads();
+        for (int i = z0*cc.H*8 + threadIdx.x; i < z1*cc.H*8; i += NT) {
+            const int z = i/(8*cc.H), y = y0 + (i/8) % cc.H, fl = kind_flag(i & 7), r = z*k.NYD6 + y + 3;
+            if (y < NY && T.bfl_flag[fl*nb + r] == 1 && T.bfl_q[fl*nb + r] < C(0.5)) list[atomicAdd(&count, 1)] = (unsigned short)i;
+        }
+        __syncthreads();
+        const int items = count*WH;
+        for (int i = threadIdx.x; i < items; i += NT) {
+            const int e = list[i/WH], xx = i % WH, kd = e & 7, fl = kind_flag(kd), q = kind_src(kd);
+            const int z = e/(8*cc.H), y = y0 + (e/8) % cc.H, r = z*k.NYD6 + y + 3;
+            const int iy = k.bfl_mode ? r : y + 3;   // reference: Y weights at [j]
+            const S *b = fo + (size_t)q*N + wrap_any(x0 + xx - 3, NX);
+            const C rq = ref(q);
+            C wy[7], sum = 0;
+#pragma unroll
+            for (int j = 0; j < 7; j++) wy[j] = bw(kind_yset(fl), j, iy);
+#pragma unroll
+            for (int c = 0; c < 7; c++) {
+                C in = 0;
+#pragma unroll
+                for (int j = 0; j < 7; j++) in += full(b + ((size_t)c*NY + wrap_near(y - 3 + j, NY))*NX, rq)*wy[j];
+                sum += in*bw(kind_zset(fl), c, r);
+            }
+            bf[(size_t)e*WH + xx] = sum;
+        }
+    }
+
+    __device__ __forceinline__ void bfl_apply(C (&F)[19], const Col &L, int z, const C *bf) const {
+        const int NX = k.NX, NY = k.NY, nb = 2*k.NYD6, WH = cc.W + 6;
+        const size_t N = (size_t)NX*NY*k.NZ;
+        const int r = z*k.NYD6 + L.y + 3;
+        const int ix = k.bfl_mode ? r : L.x + 3;   // reference: X weights at [i]
+        const S *nd = fo + ((size_t)z*NY + L.y)*NX + L.x;
+        const C *row = bf + (size_t)(z*cc.H + L.yl)*8*WH + L.xl;
+        auto lin = [&](C q, int a, int b) -> C {   // (1/(2Q)) f_a + ((2Q-1)/(2Q)) f_b at the node
+            return (C(1)/(C(2)*q))*full(nd + a*N, ref(a)) + ((C(2)*q - C(1))/(C(2)*q))*full(nd + b*N, ref(b));
+        };
+        auto xf = [&](int kd, int set) -> C {
+            C s = 0;
+#pragma unroll
+            for (int a = 0; a < 7; a++) s += bw(set, a, ix)*row[kd*WH + a];
+            return s;
+        };
+        auto at = [&](int kd) -> C { return row[kd*WH + 3]; };
+        if (T.bfl_flag[0*nb + r] == 1) {
+            const C q = T.bfl_q[0*nb + r];
+            if (q > C(0.5)) { F[3] = lin(q, 4, 3); F[7] = lin(q, 10, 7); F[8] = lin(q, 9, 8); }
+            if (q < C(0.5)) { F[3] = at(4); F[7] = xf(0, B_XB37); F[8] = xf(1, B_XB38); }
+        }
+        if (T.bfl_flag[1*nb + r] == 1) {
+            const C q = T.bfl_q[1*nb + r];
+            if (q > C(0.5)) { F[4] = lin(q, 3, 4); F[9] = lin(q, 8, 9); F[10] = lin(q, 7, 10); }
+            if (q < C(0.5)) { F[4] = at(5); F[9] = xf(2, B_XB49); F[10] = xf(3, B_XB410); }
+        }
+        if (T.bfl_flag[2*nb + r] == 1) {
+            const C q = T.bfl_q[2*nb + r];
+            if (q > C(0.5)) F[15] = lin(q, 18, 15);
+            if (q < C(0.5)) F[15] = at(6);
+        }
+        if (T.bfl_flag[3*nb + r] == 1) {
+            const C q = T.bfl_q[3*nb + r];
+            if (q > C(0.5)) F[16] = lin(q, 17, 16);
+            if (q < C(0.5)) F[16] = at(7);
+        }
+    }
+
+    // phase C: target plane t of one column
+    __device__ __forceinline__ void target(const Col &L, const Quad<C> *ring, int t, const C *bf, C f6, C f12, C rho_mod,
+                                           double &ub, double &mass) const {
+        const int NX = k.NX, NY = k.NY;
+        const size_t N = (size_t)NX*NY*k.NZ;
+        const int b = base(t);
+        C F[19];
+        {
+            C a[16];
+#pragma unroll
+            for (int j = 0; j < 16; j++) a[j] = 0;
+            const Quad<C> *w = (const Quad<C> *)(T.wxi + ((size_t)t*NY + L.y)*64);
+            int slot = b % RING;
+#pragma unroll
+            for (int c = 0; c < 7; c++) {
+                const Quad<C> w0 = w[2*c], w1 = w[2*c + 1];   // xi 3, 4, 5, 6 | 15, 16, 17, 18
+                const Quad<C> *v = ring + (size_t)slot*4*P;
+                const Quad<C> v0 = v[0], v1 = v[P], v2 = v[2*P], v3 = v[3*P];
+                a[0] += w0.a*v0.a; a[1] += w0.b*v0.b; a[2] += w0.c*v0.c; a[3] += w0.d*v0.d;
+                a[4] += w0.a*v1.a; a[5] += w0.a*v1.b; a[6] += w0.b*v1.c; a[7] += w0.b*v1.d;
+                a[8] += w0.c*v2.a; a[9] += w0.c*v2.b; a[10] += w0.d*v2.c; a[11] += w0.d*v2.d;
+                a[12] += w1.a*v3.a; a[13] += w1.b*v3.b; a[14] += w1.c*v3.c; a[15] += w1.d*v3.d;
+                slot = slot == RING - 1 ? 0 : slot + 1;
+            }
+#pragma unroll
+            for (int j = 0; j < 16; j++) F[3 + j] = a[j];
+        }
+        const size_t node = ((size_t)t*NY + L.y)*NX + L.x;
+        {
+            const S *r = fo + (size_t)t*NY*NX + L.yo[3];
+            C s1 = 0, s2 = 0;
+#pragma unroll
+            for (int a = 0; a < 7; a++) { s1 += wx0(a, L.x)*val(r + L.xo[a] + N); s2 += wx2(a, L.x)*val(r + L.xo[a] + 2*N); }
+            F[1] = s1; F[2] = s2;
+            F[0] = val(fo + node);
+        }
+        if constexpr (Storage<S>::dev) {
+#pragma unroll
+            for (int q = 0; q < 19; q++) F[q] = F[q] + ref(q);
+        }
+        const S *nd = fo + node;
+        auto opp = [&](int q) -> C { return full(nd + q*N, ref(q)); };
+        if (t == 0) { F[5] = opp(6); F[11] = opp(14); F[12] = opp(13); F[15] = opp(18); F[16] = opp(17); }
+        if (t == k.NZ - 1) { F[6] = opp(5); F[13] = opp(12); F[14] = opp(11); F[17] = opp(16); F[18] = opp(15); }
+        if (t <= 1) bfl_apply(F, L, t, bf);
+        C rho, u1, v1, w1;
+        collide_pairs<C, LES>(F, rho_mod, f6, f12, (C)k.tau, (C)k.les_C, rho, u1, v1, w1);
+#pragma unroll
+        for (int q = 0; q < 19; q++) store_f<S>(fn + (size_t)q*N, node, q, F[q]);
+        if (macros_on) { rho_out[node] = rho; u_out[node] = u1; v_out[node] = v1; w_out[node] = w1; }
+        if (L.y == k.yplane) ub += (double)v1*T.dxv[L.x]*T.dzv[t];
+        if (mass_on) mass += (double)rho;
+        if (!(rho == rho)) ctrl->nonfinite = 1u;
+    }
+
+    __device__ __forceinline__ void run(unsigned char *smem) const {
+        Quad<C> *ring = (Quad<C> *)smem;
+        Quad<C> *qb = (Quad<C> *)(smem + ring_bytes<C>());
+        const int tid = threadIdx.x, c = tid % P, g = tid/P;
+        const int WH = cc.W + 6, NX = k.NX, NY = k.NY, NZ = k.NZ;
+        double ub = 0.0, mass = 0.0;
+        const double force = ctrl->force;
+        const C f6 = (C)(1.0/6*force*k.dt), f12 = (C)(1.0/12*force*k.dt), rho_mod = (C)ctrl->rho_modify;
+        const int ntiles = cc.tiles_x*cc.tiles_y;
+        for (int item = blockIdx.x; item < ntiles*cc.segs; item += gridDim.x) {
+            const int seg = item/ntiles, tile = item - seg*ntiles;
+            const int ty = tile/cc.tiles_x, x0 = (tile - ty*cc.tiles_x)*cc.W, y0 = ty*cc.H;
+            const int ta = (int)((long long)seg*NZ/cc.segs), tb = (int)((long long)(seg + 1)*NZ/cc.segs);
+            Col L;
+            L.yl = c/cc.W; L.xl = c - L.yl*cc.W;
+            L.x = x0 + L.xl; L.y = y0 + L.yl;
+            L.on = L.yl < cc.H && L.x < NX && L.y < NY;
+            if (L.on) {
+#pragma unroll
+                for (int a = 0; a < 7; a++) {
+                    L.xo[a] = wrap_any(L.x - 3 + a, NX);
+                    L.yo[a] = wrap_near(L.y - 3 + a, NY)*NX;
+                }
+            }
+            int np = base(ta);   // next plane to filter
+            for (int t0 = ta; t0 < tb; t0 += CHUNK) {
+                const int t1 = min(t0 + CHUNK, tb);
+                const int pend = base(t1 - 1) + 7;
+                halo_quads(qb, np, pend - np, x0, y0);
+                __syncthreads();   // quads complete; every thread is done with the previous chunk's targets
+                if (L.on)
+                    for (int p = np + g; p < pend; p += GROUPS)
+                        filter(L, qb + (size_t)((p - np)*cc.H + L.yl)*WH + L.xl, p, ring + (size_t)(p % RING)*4*P + c);
+                np = pend;
+                __syncthreads();   // ring complete, quads free
+                if (t0 <= 1) {
+                    bfl_sums((C *)qb, t0, min(t1, 2), x0, y0);
+                    __syncthreads();
+                }
+                if (L.on)
+                    for (int t = t0 + g; t < t1; t += GROUPS)
+                        target(L, ring + c, t, (const C *)qb, f6, f12, rho_mod, ub, mass);
+                if (t0 <= 1) __syncthreads();   // the sums are read before the next chunk's quads replace them
+            }
+        }
+        end_of_step<NT>(ctrl, k, n, ub, mass, true, mass_on != 0, gridDim.x);
+    }
+};
+
+// CTAs per SM: shared memory (ring + quads) allows 3 in FP64 (about 71 KB) and 6 in FP32; registers
+// 168 and 128 per thread without spills
+template <class S> constexpr int min_ctas() { return sizeof(typename Storage<S>::C) == 8 ? 3 : 4; }
+
+template <class S, bool LES>
+__global__ void __launch_bounds__(NT, min_ctas<S>()) step_chunk_kernel(const __grid_constant__ Chunk<S, LES> K) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    K.run(smem);
+}
+
+template <class C> size_t smem_for(int W, int H) {
+    const size_t quads = (size_t)RING*H*(W + 6)*sizeof(Quad<C>), sums = (size_t)2*H*8*(W + 6)*sizeof(C);
+    return ring_bytes<C>() + std::max(quads, sums);
+}
+
+template <class S, bool LES>
+cudaError_t prepare_t(size_t smem, int *ctas) {
+    cudaError_t e = cudaFuncSetAttribute(step_chunk_kernel<S, LES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas, step_chunk_kernel<S, LES>, NT, smem);
+}
+
+template <class S, bool LES>
+cudaError_t launch_t(const StepLaunch &L) {
+    using C = typename Storage<S>::C;
+    Chunk<S, LES> K;
+    K.fo = (const S *)L.fo;
+    K.fn = (S *)L.fn;
+    K.T = *(const Tables<C> *)L.tables;
+    K.k = L.k;
+    K.cc = *(const ChunkConst *)L.chunk;
+    K.ctrl = L.ctrl;
+    K.n = L.n;
+    K.rho_out = (C *)L.macros[0]; K.u_out = (C *)L.macros[1]; K.v_out = (C *)L.macros[2]; K.w_out = (C *)L.macros[3];
+    for (int a = 0; a < 7; a++) {
+        K.ux0[a] = (C)K.cc.wx0[a]; K.ux2[a] = (C)K.cc.wx2[a];
+        K.uy0[a] = (C)K.cc.wy0[a]; K.uy2[a] = (C)K.cc.wy2[a];
+    }
+    K.macros_on = L.macros_on; K.mass_on = L.mass;
+    step_chunk_kernel<S, LES><<<K.cc.grid, NT, K.cc.smem_bytes, L.stream>>>(K);
+    return cudaGetLastError();
+}
+
+template <class F>
+cudaError_t by_kernel(int precision, bool les, F &&f) {
+    switch (precision) {
+    case ISLBM_FP64: return les ? f((double *)nullptr, std::true_type{}) : f((double *)nullptr, std::false_type{});
+    case ISLBM_FP32: return les ? f((float *)nullptr, std::true_type{}) : f((float *)nullptr, std::false_type{});
+    case ISLBM_FP16_DEV: return les ? f((__half *)nullptr, std::true_type{}) : f((__half *)nullptr, std::false_type{});
+    default: return les ? f((__nv_bfloat16 *)nullptr, std::true_type{}) : f((__nv_bfloat16 *)nullptr, std::false_type{});
+    }
+}
+
+}  // namespace
+
+cudaError_t make_chunk_const(const StepConst &k, int precision, bool les, const double *wx0, const double *wx2,
+                             const double *wy0, const double *wy2, int num_sms, ChunkConst *out) {
+    ChunkConst cc;
+    std::memset((void *)&cc, 0, sizeof(cc));
+    for (int a = 0; a < 7; a++) { cc.wx0[a] = wx0[a]; cc.wx2[a] = wx2[a]; cc.wy0[a] = wy0[a]; cc.wy2[a] = wy2[a]; }
+    // tile shape: the split of a row into equal parts of at most 32 columns, H rows of it, with the
+    // fewest warps per node; a part costs 32 lanes in phases B and C (about 0.95 of the work)
+    // and its halo columns in phase A
+    double best = 1e300;
+    for (int parts = (k.NX + P - 1)/P; parts <= k.NX; parts++) {
+        const int W = (k.NX + parts - 1)/parts, tx = (k.NX + W - 1)/W;
+        const int H = std::min(P/W, k.NY), ty = (k.NY + H - 1)/H;
+        const double cost = (double)tx*ty*(0.95*P + 0.05*H*(W + 6));
+        if (cost < best*(1.0 - 1e-9)) { best = cost; cc.W = W; cc.H = H; cc.tiles_x = tx; cc.tiles_y = ty; }
+        if (W <= 4) break;
+    }
+    cc.smem_bytes = precision == ISLBM_FP64 ? smem_for<double>(cc.W, cc.H) : smem_for<float>(cc.W, cc.H);
+    int ctas = 0;
+    cudaError_t e = by_kernel(precision, les, [&](auto *s, auto l) {
+        using S = std::remove_pointer_t<decltype(s)>;
+        return prepare_t<S, decltype(l)::value>(cc.smem_bytes, &ctas);
+    });
+    if (e != cudaSuccess) return e;
+    if (ctas < 1) return cudaErrorInvalidConfiguration;
+    // wall-normal segments: rounds of items x (targets per segment + the ramp of 6 planes, whose
+    // filters cost a quarter of a whole plane in FP64 and about half in FP32), down to one target
+    // where a grid has few tiles
+    const int tiles = cc.tiles_x*cc.tiles_y, slots = ctas*num_sms;
+    const double ramp = precision == ISLBM_FP64 ? 1.5 : 3.0;
+    double best_cost = 1e300;
+    for (int z = 1; z <= k.NZ; z++) {
+        const long long items = (long long)tiles*z;
+        const double rounds = (double)((items + slots - 1)/slots);
+        const double cost = rounds*((double)((k.NZ + z - 1)/z) + ramp);
+        if (cost < best_cost - 1e-9) { best_cost = cost; cc.segs = z; }
+    }
+    cc.grid = (int)std::min<long long>((long long)tiles*cc.segs, slots);
+    *out = cc;
+    return cudaSuccess;
+}
+
+cudaError_t launch_step_chunk(const StepLaunch &L) {
+    return by_kernel(L.precision, L.les, [&](auto *s, auto l) {
+        using S = std::remove_pointer_t<decltype(s)>;
+        return launch_t<S, decltype(l)::value>(L);
+    });
+}
+
+}  // namespace islbm

@@ -20,6 +20,7 @@ struct StepLaunch {
     void *macros[4];           // rho, u, v, w (compute type) when macros_on
     const void *tiled;         // TiledConst for the tiled kernel
     const void *pmaps;         // paired kernel: the 4 tensor maps (CUtensorMap) of buffer fo, or null
+    const void *chunk;         // ChunkConst for the chunk-marching kernel
     cudaStream_t stream;
 };
 

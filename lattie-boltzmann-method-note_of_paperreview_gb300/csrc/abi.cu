@@ -433,6 +433,7 @@ int init_impl(const islbm_params *pp, islbm_handle *h) {
     h->steps = 0;
     h->use_tiled = false;
     h->paired = false;
+    h->roles = false;
     h->chunked = false;
     int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
@@ -442,13 +443,19 @@ int init_impl(const islbm_params *pp, islbm_handle *h) {
         wy0[a] = h->g.YP0[(size_t)a*h->g.NYD6 + 3]; wy2[a] = h->g.YP2[(size_t)a*h->g.NYD6 + 3];
     }
     if (p.kernel == ISLBM_KERNEL_TILED || p.kernel == ISLBM_KERNEL_AUTO || p.kernel == ISLBM_KERNEL_TILED_SINGLE) {
-        // the paired-node kernel where the grid allows it, else the one-node-per-thread kernel
-        if (p.kernel != ISLBM_KERNEL_TILED_SINGLE && pair_supported(k, p.precision) &&
+        // the role-specialised paired kernel where the grid allows it, else the paired one, else the
+        // one-node-per-thread kernel; tensor-map plane copies unless the bulk row copies are asked
+        // for (comparison runs)
+        const char *cp = std::getenv("ISLBM_PAIR_COPIES");
+        const bool maps = !(cp && std::strcmp(cp, "bulk") == 0);
+        if (p.kernel != ISLBM_KERNEL_TILED_SINGLE && roles_supported(k, p.precision)) {
+            CK(make_roles_const(k, p.precision, p.les_cs > 0.0, wx0, wx2, wy0, wy2, sms, &h->tiled));
+            h->use_tiled = h->paired = h->roles = true;
+            if (maps) make_role_maps(k, (int)h->elem, h->fbuf, &h->rmaps);
+        } else if (p.kernel != ISLBM_KERNEL_TILED_SINGLE && pair_supported(k, p.precision) &&
             make_pair_const(k, p.precision, wx0, wx2, wy0, wy2, sms, &h->tiled) == 0) {
             h->use_tiled = h->paired = true;
-            // tensor-map plane copies unless the bulk row copies are asked for (comparison runs)
-            const char *cp = std::getenv("ISLBM_PAIR_COPIES");
-            if (!(cp && std::strcmp(cp, "bulk") == 0)) make_pair_maps(k, (int)h->elem, h->fbuf, &h->pmaps);
+            if (maps) make_pair_maps(k, (int)h->elem, h->fbuf, &h->pmaps);
         } else if (tiled_supported(k, p.precision) && make_tiled_const(k, p.precision, wx0, wx2, wy0, wy2, sms, &h->tiled) == 0) {
             h->use_tiled = true;
         }
@@ -530,12 +537,12 @@ int islbm_step(islbm_handle *h, int nsteps) {
         const unsigned long long n = h->steps + 1;
         L.fo = h->fbuf[h->cur];
         L.fn = h->fbuf[1 - h->cur];
-        L.pmaps = h->paired ? h->pmaps.for_buffer(L.fo) : nullptr;
+        L.pmaps = h->roles ? h->rmaps.for_buffer(L.fo) : h->paired ? h->pmaps.for_buffer(L.fo) : nullptr;
         L.n = n;
         L.mass = h->p.mass_interval > 0 && (n % (unsigned long long)h->p.mass_interval) == 0ULL;
         L.macros_on = (s == nsteps - 1);
         for (int m = 0; m < 4; m++) L.macros[m] = h->macros[m];
-        cudaError_t e = h->paired ? launch_step_pair(L) : h->use_tiled ? launch_step_tiled(L) : h->chunked ? launch_step_chunk(L) : launch_step_gather(L);
+        cudaError_t e = h->roles ? launch_step_roles(L) : h->paired ? launch_step_pair(L) : h->use_tiled ? launch_step_tiled(L) : h->chunked ? launch_step_chunk(L) : launch_step_gather(L);
         if (e != cudaSuccess) return cuda_fail(e, "step kernel launch");
         h->cur = 1 - h->cur;
         h->steps = n;

@@ -39,6 +39,8 @@ struct islbm_handle {
 
     double *xfer = nullptr;    // FP64 transfer buffer of N values for host copies (first use)
     TiledConst tiled{};
+    bool roles = false;        // ... with paired: the role-specialised kernel (step_roles.cuh)
+    RoleMaps rmaps{};
     bool chunked = false;      // the chunk-marching kernel (step_chunk.cu) steps this solve
     ChunkConst chunk{};
     PairMaps pmaps{};          // tensor maps of fbuf[0], fbuf[1] for the paired kernel's copies

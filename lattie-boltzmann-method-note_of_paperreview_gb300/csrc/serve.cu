@@ -110,6 +110,7 @@ struct Group {
     int precision = 0, NX = 0;
     bool les = false;
     bool paired = false;         // members step with the paired-node kernel (step_pair.cu)
+    bool roles = false;          // ... the role-specialised one (step_roles.cuh)
     std::vector<Solve *> members;
     void *descs = nullptr;       // device descriptors
     int2 *items = nullptr;       // device (solve, segment*ntiles + tile) work list
@@ -248,7 +249,7 @@ int build_groups(islbm_server *s, std::vector<Group *> &out, std::vector<Solve *
         islbm_handle *h = v->h;
         if (!h->use_tiled) { singles.push_back(v); continue; }
         const std::string sig = std::to_string(h->p.precision) + "/" + std::to_string(h->p.NX) + "/" +
-                                std::to_string(h->p.les_cs > 0.0 ? 1 : 0) + "/" + std::to_string(h->paired ? 1 : 0);
+                                std::to_string(h->p.les_cs > 0.0 ? 1 : 0) + "/" + std::to_string(h->roles ? 2 : h->paired ? 1 : 0);
         by[sig].push_back(v);
     }
     for (auto &kv : by) {
@@ -259,17 +260,17 @@ int build_groups(islbm_server *s, std::vector<Group *> &out, std::vector<Solve *
         if (it != s->groups.end()) { free_group(it->second.get()); s->groups.erase(it); }
         auto g = std::make_unique<Group>();
         islbm_handle *h0 = kv.second[0]->h;
-        g->precision = h0->p.precision; g->NX = h0->p.NX; g->les = h0->p.les_cs > 0.0; g->paired = h0->paired;
+        g->precision = h0->p.precision; g->NX = h0->p.NX; g->les = h0->p.les_cs > 0.0; g->paired = h0->paired; g->roles = h0->roles;
         g->members = kv.second;
         g->key = key;
-        const size_t db = g->paired ? pair_batch_desc_bytes(g->precision, g->NX, g->les)
+        const size_t db = g->roles ? roles_batch_desc_bytes(g->precision, g->NX, g->les) : g->paired ? pair_batch_desc_bytes(g->precision, g->NX, g->les)
                                     : batch_desc_bytes(g->precision, g->NX, g->les);
         std::vector<unsigned char> hd(db*g->members.size());
         std::vector<int2> items;
         int maxt = 0, total_tiles = 0, min_nz = 1 << 30;
         for (size_t m = 0; m < g->members.size(); m++) {
             islbm_handle *h = g->members[m]->h;
-            const int ntiles = h->p.NY/h->tiled.TY;
+            const int ntiles = (h->p.NY + h->tiled.TY - 1)/h->tiled.TY;
             maxt = std::max(maxt, ntiles);
             total_tiles += ntiles;
             min_nz = std::min(min_nz, h->p.NZ);
@@ -277,13 +278,21 @@ int build_groups(islbm_server *s, std::vector<Group *> &out, std::vector<Solve *
         // wall-normal segments per column: enough work items for four CTAs per SM, each segment
         // at least 16 targets long (a segment re-reads the 6 planes below it to fill its ring)
         // (paired kernel: two CTAs per SM, segment count by the makespan estimate of pair_zsegs)
-        const int nseg = g->paired ? pair_zsegs(total_tiles, 2*s->sms, min_nz)
+        const int nseg = g->roles ? roles_segments(total_tiles, s->sms, min_nz) : g->paired ? pair_zsegs(total_tiles, 2*s->sms, min_nz)
                                    : std::max(1, std::min(4*s->sms/std::max(1, total_tiles), min_nz/16));
         for (size_t m = 0; m < g->members.size(); m++) {
             islbm_handle *h = g->members[m]->h;
             g->nodes += (long long)h->N;
+            const int nt = (h->p.NY + h->tiled.TY - 1)/h->tiled.TY;
+            if (g->roles) {
+                RoleMaps maps;   // as the handle's own, made for its buffers
+                if (h->rmaps.ok) maps = h->rmaps;
+                fill_roles_batch_desc(g->precision, g->NX, g->les, h->tf, h->k, h->tiled, h->ctrl, h->macros, h->fbuf, maps, nt, nseg,
+                                      hd.data() + m*db);
+                continue;
+            }
             (g->paired ? fill_pair_batch_desc : fill_batch_desc)(g->precision, g->NX, g->les, h->tf, h->k, h->tiled, h->ctrl, h->macros, h->fbuf[0], h->fbuf[1],
-                            h->p.NY/h->tiled.TY, nseg, hd.data() + m*db);
+                            nt, nseg, hd.data() + m*db);
         }
         // segment-major, the solves' tiles interleaved, so that neighbouring tiles of a solve at
         // the same height run together
@@ -291,7 +300,7 @@ int build_groups(islbm_server *s, std::vector<Group *> &out, std::vector<Solve *
             for (int t = 0; t < maxt; t++)
                 for (size_t m = 0; m < g->members.size(); m++) {
                     islbm_handle *h = g->members[m]->h;
-                    const int nt = h->p.NY/h->tiled.TY;
+                    const int nt = (h->p.NY + h->tiled.TY - 1)/h->tiled.TY;
                     if (t < nt) items.push_back(make_int2((int)m, seg*nt + t));
                 }
         g->nitems = (int)items.size();
@@ -315,6 +324,8 @@ int build_groups(islbm_server *s, std::vector<Group *> &out, std::vector<Solve *
 
 // one batched step of every member of g on the group's stream
 cudaError_t launch_batch(Group *g, int grid, int macros_on) {
+    if (g->roles)
+        return launch_step_roles_batch(g->precision, g->NX, g->les, g->descs, g->items, g->nitems, grid, macros_on, g->stream);
     return g->paired ? launch_step_pair_batch(g->precision, g->NX, g->les, g->descs, g->items, g->nitems, grid, macros_on, g->stream)
                      : launch_step_tiled_batch(g->precision, g->NX, g->les, g->descs, g->items, g->nitems, grid, macros_on, g->stream);
 }
@@ -362,7 +373,7 @@ int run_group_chunk(islbm_server *s, Group *g, int steps) {
         if (g->graph) cudaGraphExecDestroy(g->graph);
         g->graph = nullptr;
         cudaGraph_t graph;
-        SK(g->paired ? prepare_step_pair_batch(g->precision, g->NX, g->les) : prepare_step_tiled_batch(g->precision, g->NX, g->les));
+        if (!g->roles) SK(g->paired ? prepare_step_pair_batch(g->precision, g->NX, g->les) : prepare_step_tiled_batch(g->precision, g->NX, g->les));
         SK(cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal));
         for (int j = 0; j < steps; j++) {
             cudaError_t e = launch_batch(g, g->grid, j == steps - 1);

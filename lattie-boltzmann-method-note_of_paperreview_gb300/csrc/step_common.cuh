@@ -233,7 +233,8 @@ __device__ __forceinline__ double warp_sum(double v) {
 // End-of-step bookkeeping, run by the last block of the step kernel (after every block has
 // added its partial sums): bulk-velocity window, forcing controller every NDTFRC steps
 // (C/evolution.h:1003-1042) and the mass correction for the next step.
-__device__ __forceinline__ void finish_step(Ctrl *ctrl, const StepConst &k, unsigned long long n, bool mass_step) {
+// `mass`: the sum of the mass slots on a mass-check step.
+__device__ __forceinline__ void finish_step(Ctrl *ctrl, const StepConst &k, unsigned long long n, bool mass_step, double mass) {
     // other blocks updated these with atomics during this kernel: read them from L2
     double acc = __ldcg(&ctrl->ub_acc) + __ldcg(&ctrl->ub_slot[(n - 1) & 1]);
     ctrl->ub_slot[(n - 1) & 1] = 0.0;
@@ -246,10 +247,8 @@ __device__ __forceinline__ void finish_step(Ctrl *ctrl, const StepConst &k, unsi
     ctrl->ub_acc = acc;
     ctrl->force = force;
     if (mass_step) {
-        double m = 0.0;
-        for (int i = 0; i < 256; i++) { m += __ldcg(&ctrl->mass_slot[i]); ctrl->mass_slot[i] = 0.0; }
-        ctrl->rho_modify = (k.nnodes - m)/k.nnodes;
-        if (!(m == m)) ctrl->nonfinite = 1u;
+        ctrl->rho_modify = (k.nnodes - mass)/k.nnodes;
+        if (!(mass == mass)) ctrl->nonfinite = 1u;
     } else {
         ctrl->rho_modify = 0.0;
     }
@@ -300,8 +299,42 @@ __device__ __forceinline__ void end_of_step(Ctrl *ctrl, const StepConst &k, unsi
     __syncthreads();
     if (last && tid == 0) {
         __threadfence();
-        finish_step(ctrl, k, n, mass_step);
+        double m = 0.0;
+        if (mass_step)
+            for (int i = 0; i < 256; i++) { m += __ldcg(&ctrl->mass_slot[i]); ctrl->mass_slot[i] = 0.0; }
+        finish_step(ctrl, k, n, mass_step, m);
     }
+}
+
+// The same for a group of NTHREADS threads (a multiple of 32, `tid` = 0 .. NTHREADS - 1) of a larger
+// block, synchronised by `sync`.
+template <int NTHREADS, class SYNC>
+__device__ __forceinline__ void end_of_step_group(Ctrl *ctrl, const StepConst &k, unsigned long long n, double ub, double mass,
+                                                  bool mass_step, unsigned total, int tid, SYNC &&sync) {
+    __shared__ double gred[2][NTHREADS/32];
+    __shared__ bool glast;
+    const int lane = tid & 31, warp = tid >> 5;
+    ub = warp_sum(ub);
+    if (mass_step) mass = warp_sum(mass);
+    if (lane == 0) { gred[0][warp] = ub; gred[1][warp] = mass; }
+    sync();
+    if (tid == 0) {
+        double s = 0.0, m = 0.0;
+        for (int w = 0; w < NTHREADS/32; w++) { s += gred[0][w]; m += gred[1][w]; }
+        if (s != 0.0) atomicAdd(&ctrl->ub_slot[n & 1ULL], s);   // (also a NaN)
+        if (mass_step) atomicAdd(&ctrl->mass_slot[blockIdx.x & 255u], m);
+        __threadfence();
+        glast = atomicAdd(&ctrl->done, 1u) == total - 1u;
+    }
+    sync();
+    if (!glast || tid >= 32) return;
+    __threadfence();
+    double m = 0.0;
+    if (mass_step) {   // the 256 mass slots, summed by one warp
+        for (int i = lane; i < 256; i += 32) { m += __ldcg(&ctrl->mass_slot[i]); ctrl->mass_slot[i] = 0.0; }
+        m = warp_sum(m);
+    }
+    if (lane == 0) finish_step(ctrl, k, n, mass_step, m);
 }
 
 }  // namespace islbm

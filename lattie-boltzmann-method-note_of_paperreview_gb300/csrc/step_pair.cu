@@ -43,6 +43,7 @@
 #include "step_launch.hpp"
 #include "step_tiled.hpp"
 #include "tile_helpers.cuh"
+#include "pair_helpers.cuh"
 
 namespace islbm {
 
@@ -121,74 +122,6 @@ struct PLay {
 // F1 pair, F2 pair.
 __device__ __forceinline__ uint32_t pring_col(int slot) { return 32u*(uint32_t)slot; }
 __device__ __forceinline__ uint32_t pdelay_col(int p) { return 224u + 4u*(uint32_t)(p & 7); }
-
-__device__ __forceinline__ void tmem_st16(uint32_t ta, const float (&v)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(ta),
-        "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]),
-        "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15])
-        : "memory");
-}
-__device__ __forceinline__ void tmem_st4(uint32_t ta, float a, float b, float c, float d) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(ta), "f"(a), "f"(b), "f"(c), "f"(d)
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t ta, uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-          "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-          "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(ta)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_ld4(uint32_t ta, uint32_t (&v)[4]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
-                 : "r"(ta)
-                 : "memory");
-}
-
-// two stored values of adjacent nodes -> FP32 pair (the deviation formats give deviations)
-template <class S> __device__ __forceinline__ V2 ld2v(const S *p);
-template <> __device__ __forceinline__ V2 ld2v<float>(const float *p) { return V2(*(const float2 *)p); }
-template <> __device__ __forceinline__ V2 ld2v<__half>(const __half *p) { return V2(__half22float2(*(const __half2 *)p)); }
-template <> __device__ __forceinline__ V2 ld2v<__nv_bfloat16>(const __nv_bfloat16 *p) {
-    return V2(__bfloat1622float2(*(const __nv_bfloat162 *)p));
-}
-// full values of a node pair from global memory (read-only path)
-template <class S> __device__ __forceinline__ V2 ld2g(const S *p, int q) {
-    V2 v;
-    if constexpr (std::is_same<S, float>::value) v = V2(__ldg((const float2 *)p));
-    else if constexpr (std::is_same<S, __half>::value) {
-        const unsigned r = __ldg((const unsigned *)p);
-        v = V2(__half22float2(*(const __half2 *)&r));
-    } else {
-        const unsigned r = __ldg((const unsigned *)p);
-        v = V2(__bfloat1622float2(*(const __nv_bfloat162 *)&r));
-    }
-    if constexpr (Storage<S>::dev) v = v + V2((float)dev_ref(q));
-    return v;
-}
-// store a node pair (full values; the deviation formats store f - ref)
-template <class S> __device__ __forceinline__ void st2(S *p, V2 v, int q) {
-    if constexpr (std::is_same<S, float>::value) *(float2 *)p = v.v;
-    else {
-        const V2 d = v - V2((float)dev_ref(q));
-        if constexpr (std::is_same<S, __half>::value) *(__half2 *)p = __float22half2_rn(d.v);
-        else *(__nv_bfloat162 *)p = __float22bfloat162_rn(d.v);
-    }
-}
-
-// Tensor copy of one box (x, y, z, q) of a population buffer: the box lands in shared memory as
-// [q][rows][NX], the layout of the front and stage buffers.
-__device__ __forceinline__ void tma_load4(void *dst, const CUtensorMap *map, int x, int y, int z, int q, uint64_t *bar) {
-    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
-                 ::"r"(smem_u32(dst)), "l"((unsigned long long)map), "r"(x), "r"(y), "r"(z), "r"(q), "r"(smem_u32(bar))
-                 : "memory");
-}
 
 // The four tensor maps of the buffer a launch reads (kernel parameter: tensor maps must live in
 // parameter, constant or global memory)
@@ -890,13 +823,9 @@ int pair_zsegs(int tiles, int slots, int NZ) {
     return best;
 }
 
-int make_pair_const(const StepConst &k, int precision, const double *wx0, const double *wx2, const double *wy0,
-                    const double *wy2, int num_sms, TiledConst *out) {
-    TiledConst tc;
-    std::memset(&tc, 0, sizeof(tc));
-    const PLayInfo li = precision == ISLBM_FP32 ? play_for<float>(k.NX) : play_for<__half>(k.NX);
-    tc.TY = li.ty;
-    tc.smem_bytes = li.smem;
+int fill_pair_weights(const double *wx0, const double *wx2, const double *wy0, const double *wy2, TiledConst *out) {
+    TiledConst &tc = *out;
+    std::memset((void *)&tc, 0, sizeof(tc));
     for (int a = 0; a < 7; a++) {
         tc.wx[a] = make_float2((float)wx0[a], (float)wx2[a]);
         tc.wy[a] = make_float2((float)wy0[a], (float)wy2[a]);
@@ -916,6 +845,16 @@ int make_pair_const(const StepConst &k, int precision, const double *wx0, const 
             tc.wxb[set][kk] = make_float2(W(ky + 2), W(ky + 3));
         }
     }
+    return 0;
+}
+
+int make_pair_const(const StepConst &k, int precision, const double *wx0, const double *wx2, const double *wy0,
+                    const double *wy2, int num_sms, TiledConst *out) {
+    TiledConst tc;
+    fill_pair_weights(wx0, wx2, wy0, wy2, &tc);
+    const PLayInfo li = precision == ISLBM_FP32 ? play_for<float>(k.NX) : play_for<__half>(k.NX);
+    tc.TY = li.ty;
+    tc.smem_bytes = li.smem;
     const int tiles = k.NY/tc.TY;
     const int per_sm = (int)std::min<size_t>((size_t)li.ctas_per_sm, (228*1024)/(tc.smem_bytes + 1024));
     const int slots = per_sm*num_sms;
@@ -929,10 +868,8 @@ int make_pair_const(const StepConst &k, int precision, const double *wx0, const 
     return tc.smem_bytes <= 227*1024 ? 0 : -1;
 }
 
-bool make_pair_maps(const StepConst &k, int elem_bytes, void *const buf[2], PairMaps *out) {
-    out->ok = false;
-    if ((elem_bytes != 4 && elem_bytes != 2) || k.NX > 256 || !pair_supported(k, elem_bytes == 4 ? ISLBM_FP32 : ISLBM_FP16_DEV))
-        return false;
+// Tensor map of a population buffer over (x, y, z, q); the driver's encoder checks it
+bool encode_population_map(CUtensorMap *out, const StepConst &k, int elem_bytes, void *buf, const unsigned (&box)[4]) {
     // the driver's encoder, looked up once (thread-safe static initialisation)
     static const PFN_cuTensorMapEncodeTiled_v12000 encode = []() -> PFN_cuTensorMapEncodeTiled_v12000 {
         void *fn = nullptr;
@@ -943,19 +880,24 @@ bool make_pair_maps(const StepConst &k, int elem_bytes, void *const buf[2], Pair
         return (PFN_cuTensorMapEncodeTiled_v12000)fn;
     }();
     if (!encode) return false;
-    const int TY = 256/k.NX;   // rows per tile of the paired layout (128 threads, two nodes each)
     const size_t es = (size_t)elem_bytes;
     const cuuint64_t dims[4] = {(cuuint64_t)k.NX, (cuuint64_t)k.NY, (cuuint64_t)k.NZ, 19};
     const cuuint64_t strides[3] = {k.NX*es, (size_t)k.NX*k.NY*es, (size_t)k.NX*k.NY*k.NZ*es};
-    const cuuint32_t boxes[4][4] = {{(cuuint32_t)k.NX, (cuuint32_t)TY + 6, 1, 2}, {(cuuint32_t)k.NX, (cuuint32_t)TY + 6, 1, 4},
-                                    {(cuuint32_t)k.NX, (cuuint32_t)TY, 1, 2}, {(cuuint32_t)k.NX, (cuuint32_t)TY, 1, 4}};
     const cuuint32_t unit[4] = {1, 1, 1, 1};
     const CUtensorMapDataType dt = elem_bytes == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16;
+    return encode(out, dt, 4, buf, dims, strides, box, unit, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+bool make_pair_maps(const StepConst &k, int elem_bytes, void *const buf[2], PairMaps *out) {
+    out->ok = false;
+    if ((elem_bytes != 4 && elem_bytes != 2) || k.NX > 256 || !pair_supported(k, elem_bytes == 4 ? ISLBM_FP32 : ISLBM_FP16_DEV))
+        return false;
+    const cuuint32_t TY = (cuuint32_t)(256/k.NX), NX = (cuuint32_t)k.NX;   // rows per tile of the paired layout
+    const cuuint32_t boxes[4][4] = {{NX, TY + 6, 1, 2}, {NX, TY + 6, 1, 4}, {NX, TY, 1, 2}, {NX, TY, 1, 4}};
     for (int b = 0; b < 2; b++)
         for (int j = 0; j < 4; j++)
-            if (encode(&out->m[b][j], dt, 4, buf[b], dims, strides, boxes[j], unit, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                       CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-                return false;
+            if (!encode_population_map(&out->m[b][j], k, elem_bytes, buf[b], boxes[j])) return false;
     out->buf[0] = buf[0];
     out->buf[1] = buf[1];
     out->ok = true;

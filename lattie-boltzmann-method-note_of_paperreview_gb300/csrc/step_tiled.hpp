@@ -24,6 +24,9 @@ struct TiledConst {
     // node 1 (wxb), set 0 = wx0, set 1 = wx2
     float2 wyb[2][7];
     float2 wxa[2][4], wxb[2][4];
+    // role-specialised kernel (step_roles.cu): zmain segments of zlen targets from the bottom of every
+    // column, the rest of the column in zsegs equal ones
+    int zmain, zlen;
     unsigned long long n;         // step number (set per launch)
 };
 
@@ -70,5 +73,34 @@ void fill_pair_batch_desc(int precision, int NX, bool les, const Tables<float> &
 cudaError_t prepare_step_pair_batch(int precision, int NX, bool les);
 cudaError_t launch_step_pair_batch(int precision, int NX, bool les, const void *descs, const int2 *items, int nitems,
                                    int grid, int macros_on, cudaStream_t stream);
+
+// the weights of a TiledConst (everything else zero)
+int fill_pair_weights(const double *wx0, const double *wx2, const double *wy0, const double *wy2, TiledConst *out);
+// tensor map of a population buffer with the given box (x, y, z, population)
+bool encode_population_map(CUtensorMap *out, const StepConst &k, int elem_bytes, void *buf, const unsigned (&box)[4]);
+
+// Role-specialised paired kernel (step_roles.cu)
+struct RoleMaps {
+    CUtensorMap m[2][5];
+    const void *buf[2] = {nullptr, nullptr};
+    bool ok = false;
+    const void *for_buffer(const void *fo) const {
+        for (int b = 0; b < 2; b++)
+            if (ok && buf[b] == fo) return (const void *)m[b];
+        return nullptr;
+    }
+};
+bool roles_supported(const StepConst &k, int precision);
+// launch constants and kernel attributes on the current device
+cudaError_t make_roles_const(const StepConst &k, int precision, bool les, const double *wx0, const double *wx2,
+                             const double *wy0, const double *wy2, int num_sms, TiledConst *out);
+int roles_segments(int tiles, int slots, int NZ);   // equal segments per column for a batch of `tiles` tiles
+bool make_role_maps(const StepConst &k, int elem_bytes, void *const buf[2], RoleMaps *out);
+cudaError_t launch_step_roles(const StepLaunch &L);
+size_t roles_batch_desc_bytes(int precision, int NX, bool les);
+void fill_roles_batch_desc(int precision, int NX, bool les, const Tables<float> &T, const StepConst &k, const TiledConst &tc,
+                           Ctrl *ctrl, void *const macros[4], void *const buf[2], const RoleMaps &maps, int ntiles, int nseg, void *out);
+cudaError_t launch_step_roles_batch(int precision, int NX, bool les, const void *descs, const int2 *items, int nitems, int grid,
+                                    int macros_on, cudaStream_t stream);
 
 }  // namespace islbm

@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <cstring>
 
+#include "collide.cuh"
 #include "step_common.cuh"
 #include "step_launch.hpp"
 #include "step_chunk.hpp"
@@ -287,7 +288,7 @@ struct Chunk {
         if (t == k.NZ - 1) { F[6] = opp(5); F[13] = opp(12); F[14] = opp(11); F[17] = opp(16); F[18] = opp(15); }
         if (t <= 1) bfl_apply(F, L, t, bf);
         C rho, u1, v1, w1;
-        collide_pairs<C, LES>(F, rho_mod, f6, f12, (C)k.tau, (C)k.les_C, rho, u1, v1, w1);
+        collide<LES>(F, rho_mod, f6, f12, (C)k.tau, (C)k.les_C, rho, u1, v1, w1);
 #pragma unroll
         for (int q = 0; q < 19; q++) store_f<S>(fn + (size_t)q*N, node, q, F[q]);
         if (macros_on) { rho_out[node] = rho; u_out[node] = u1; v_out[node] = v1; w_out[node] = w1; }

@@ -542,7 +542,7 @@ struct RoleKernel {
             F[17] = ld2g<S>(b + 16*N, 16); F[18] = ld2g<S>(b + 15*N, 15);
         }
         V2 rho, u1, v1, w1;
-        collide_x2<LES>(F, sc.rho_mod, sc.f6, sc.f12, sc.tau, sc.lesC, rho, u1, v1, w1);
+        collide<LES>(F, sc.rho_mod, sc.f6, sc.f12, sc.tau, sc.lesC, rho, u1, v1, w1);
 #pragma unroll
         for (int q = 0; q < 19; q++) st2<S>(fnq[q] + node, F[q], q);
         if (macros_on) {

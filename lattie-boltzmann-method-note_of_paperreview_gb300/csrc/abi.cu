@@ -76,7 +76,7 @@ size_t tables_bytes(const islbm_params &p) {
 
 size_t required_bytes(const islbm_params &p) {
     const size_t N = (size_t)p.NX*p.NY*p.NZ;
-    return 2*19*N*storage_bytes(p.precision) + 4*N*compute_bytes(p.precision) + tables_bytes(p) + align256(sizeof(Ctrl));
+    return 2*19*N*storage_bytes(p.precision) + 4*N*compute_bytes(p.precision) + tables_bytes(p) + CTRL_BYTES;
 }
 
 // unique node (x, y, z) <-> reference index (i, j, k)
@@ -390,7 +390,8 @@ int init_impl(const islbm_params *pp, islbm_handle *h) {
     for (int m = 0; m < 4; m++) CK(cudaMalloc(&h->macros[m], h->N*h->celem));
     h->tab_bytes = tables_bytes(p);
     CK(cudaMalloc(&h->tabmem, h->tab_bytes));
-    CK(cudaMalloc(&h->ctrl, sizeof(Ctrl)));
+    CK(cudaMalloc(&h->ctrl, CTRL_BYTES));
+    CK(cudaMemsetAsync(h->ctrl, 0, CTRL_BYTES, h->stream));
 
     std::vector<char> blob;
     if (p.precision == ISLBM_FP64) pack_tables<double>(h->g, p, blob, h->td, (char *)h->tabmem);
@@ -539,6 +540,7 @@ int islbm_step(islbm_handle *h, int nsteps) {
         L.fn = h->fbuf[1 - h->cur];
         L.pmaps = h->roles ? h->rmaps.for_buffer(L.fo) : h->paired ? h->pmaps.for_buffer(L.fo) : nullptr;
         L.n = n;
+        L.launch = ++h->launches;
         L.mass = h->p.mass_interval > 0 && (n % (unsigned long long)h->p.mass_interval) == 0ULL;
         L.macros_on = (s == nsteps - 1);
         for (int m = 0; m < 4; m++) L.macros[m] = h->macros[m];

@@ -23,6 +23,7 @@
 // gather kernel, per step: FP64 256x128x192 (LES) 28.2 -> 6.97 ms, FP64 64x32x48 506 -> 135 us, FP32
 // 187x91x131 (LES) 2,956 -> 232 us (9.6 GLUPS).
 #include <algorithm>
+#include <type_traits>
 #include <cstring>
 
 #include "collide.cuh"
@@ -288,7 +289,8 @@ struct Chunk {
         if (t == k.NZ - 1) { F[6] = opp(5); F[13] = opp(12); F[14] = opp(11); F[17] = opp(16); F[18] = opp(15); }
         if (t <= 1) bfl_apply(F, L, t, bf);
         C rho, u1, v1, w1;
-        collide<LES>(F, rho_mod, f6, f12, (C)k.tau, (C)k.les_C, rho, u1, v1, w1);
+        if constexpr (std::is_same<S, float>::value) collide_pairs<C, LES>(F, rho_mod, f6, f12, (C)k.tau, (C)k.les_C, rho, u1, v1, w1);
+        else collide<LES>(F, rho_mod, f6, f12, (C)k.tau, (C)k.les_C, rho, u1, v1, w1);
 #pragma unroll
         for (int q = 0; q < 19; q++) store_f<S>(fn + (size_t)q*N, node, q, F[q]);
         if (macros_on) { rho_out[node] = rho; u_out[node] = u1; v_out[node] = v1; w_out[node] = w1; }
@@ -342,7 +344,7 @@ struct Chunk {
                 if (t0 <= 1) __syncthreads();   // the sums are read before the next chunk's quads replace them
             }
         }
-        end_of_step<NT>(ctrl, k, n, ub, mass, true, mass_on != 0, gridDim.x);
+        end_of_step_ordered<NT>(ctrl, k, n, ub, mass, mass_on != 0, blockIdx.x, gridDim.x, tid, [] { __syncthreads(); });
     }
 };
 
@@ -353,6 +355,8 @@ template <class S> constexpr int min_ctas() { return sizeof(typename Storage<S>:
 template <class S, bool LES>
 __global__ void __launch_bounds__(NT, min_ctas<S>()) step_chunk_kernel(const __grid_constant__ Chunk<S, LES> K) {
     extern __shared__ __align__(128) unsigned char smem[];
+    grid_dependency_trigger();
+    grid_dependency_wait();
     K.run(smem);
 }
 
@@ -385,8 +389,7 @@ cudaError_t launch_t(const StepLaunch &L) {
         K.uy0[a] = (C)K.cc.wy0[a]; K.uy2[a] = (C)K.cc.wy2[a];
     }
     K.macros_on = L.macros_on; K.mass_on = L.mass;
-    step_chunk_kernel<S, LES><<<K.cc.grid, NT, K.cc.smem_bytes, L.stream>>>(K);
-    return cudaGetLastError();
+    return launch_dependent(step_chunk_kernel<S, LES>, K.cc.grid, NT, K.cc.smem_bytes, L.stream, K);
 }
 
 template <class F>

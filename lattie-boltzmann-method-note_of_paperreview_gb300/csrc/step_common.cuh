@@ -82,6 +82,15 @@ struct Ctrl {
     unsigned int fault;      // set when a pipeline wait gave up (bounded waits)
 };
 
+// Behind the controller in its allocation: the seats of a step launch whose blocks choose their work by
+// the SM they run on (step_roles.cuh; the number of the last launch that took each), and the partial
+// sums (plane sum, mass) of a step's blocks or work items.
+constexpr int MAX_SEATS = 256, MAX_PARTS = 2048;
+constexpr size_t SEATS_OFF = (sizeof(Ctrl) + 255)/256*256, PARTS_OFF = SEATS_OFF + MAX_SEATS*sizeof(unsigned long long);
+constexpr size_t CTRL_BYTES = PARTS_OFF + MAX_PARTS*sizeof(double2);
+__device__ __forceinline__ unsigned long long *ctrl_seats(Ctrl *c) { return (unsigned long long *)((char *)c + SEATS_OFF); }
+__device__ __forceinline__ double2 *ctrl_parts(Ctrl *c) { return (double2 *)((char *)c + PARTS_OFF); }
+
 template <class C> struct Tables {
     const C *wx0, *wx2;        // [a*NX + x], departure x -/+ minSize
     const C *wy0, *wy2;        // [a*NY + y], departure y -/+ minSize
@@ -179,6 +188,51 @@ __device__ __forceinline__ void collide_node(C (&F)[19], C rho_modify, C f6, C f
     F[9] -= f12; F[10] -= f12; F[16] -= f12; F[18] -= f12;
 }
 
+// The operator of collide_node computed from the pair
+// sums F[a] + F[b] and differences F[a] - F[b] of the opposite directions (a, b), so that
+// density, momentum, the non-equilibrium pair sums/differences and the relaxation share them
+// (the equilibrium part of a pair is 2 w rho (1 - 1.5 u.u + 4.5 c^2) in the sum and
+// 6 w rho c in the difference, c = e_a . u). About 290 operations against 350 of collide_node.
+template <class C, bool LES>
+__device__ __forceinline__ void collide_pairs(C (&F)[19], C rho_modify, C f6, C f12, C tau, C lesC, C &rho_s, C &u1, C &v1,
+                                              C &w1) {
+    constexpr int PA[9] = {1, 3, 5, 7, 8, 11, 12, 15, 16}, PB[9] = {2, 4, 6, 10, 9, 14, 13, 18, 17};
+    F[0] = F[0] + rho_modify;
+    C S[9], A[9];
+#pragma unroll
+    for (int p = 0; p < 9; p++) { S[p] = F[PA[p]] + F[PB[p]]; A[p] = F[PA[p]] - F[PB[p]]; }
+    const C r = ((F[0] + S[0]) + (S[1] + S[2])) + ((S[3] + S[4]) + (S[5] + S[6])) + (S[7] + S[8]);
+    rho_s = r;
+    const C inv = my_rcp<C>(r);
+    u1 = ((A[0] + A[3]) + (A[5] - (A[4] + A[6])))*inv;
+    v1 = ((A[1] + A[3]) + (A[4] + (A[7] - A[8])))*inv;
+    w1 = ((A[2] + A[5]) + (A[6] + (A[7] + A[8])))*inv;
+    const C udot = u1*u1 + v1*v1 + w1*w1;
+    const C base = C(1) - C(1.5)*udot;
+    const C a1 = C(1.0/18.0)*r, a2 = C(1.0/36.0)*r;
+    const C d0 = F[0] - C(1.0/3.0)*r*base;
+    {
+        const C cu[9] = {u1, v1, w1, u1 + v1, -u1 + v1, u1 + w1, -u1 + w1, v1 + w1, -v1 + w1};
+#pragma unroll
+        for (int p = 0; p < 9; p++) {
+            const C a = p < 3 ? a1 : a2;
+            S[p] = S[p] - C(2)*a*(base + C(4.5)*cu[p]*cu[p]);
+            A[p] = A[p] - C(6)*a*cu[p];
+        }
+    }
+    C s_nu = my_rcp<C>(tau);
+    if constexpr (LES) {
+        const C Qn = pi_neq_norm2_pairs(S);
+        const C nu0 = (tau - C(0.5))*C(1.0/3.0);
+        const C Sm = my_div<C>(my_sqrt<C>(nu0*nu0 + C(18)*lesC*my_sqrt<C>(Qn)) - nu0, C(6)*lesC);
+        s_nu = my_rcp<C>(tau + C(3)*lesC*Sm);
+    }
+    mrt_relax_pairs<C>(F, d0, S, A, C(1.19), C(1.4), C(1.2), s_nu, C(1.4), C(1.5));
+    F[3] += f6; F[4] -= f6;
+    F[7] += f12; F[8] += f12; F[15] += f12; F[17] += f12;
+    F[9] -= f12; F[10] -= f12; F[16] -= f12; F[18] -= f12;
+}
+
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -261,14 +315,18 @@ __device__ __forceinline__ void end_of_step(Ctrl *ctrl, const StepConst &k, unsi
     }
 }
 
-// The same for a group of NTHREADS threads (a multiple of 32, `tid` = 0 .. NTHREADS - 1) of a larger
-// block, synchronised by `sync`.
+// The same in a fixed order, so that the controller's sums (and every result) do not depend on which
+// block comes first: block or work item `index` of `total` stores its partial sums, the last one to
+// finish adds them by index. Run by a group of NTHREADS threads (a multiple of 32, tid = 0 ..
+// NTHREADS - 1) synchronised by `sync`. More parts than MAX_PARTS are added atomically.
 template <int NTHREADS, class SYNC>
-__device__ __forceinline__ void end_of_step_group(Ctrl *ctrl, const StepConst &k, unsigned long long n, double ub, double mass,
-                                                  bool mass_step, unsigned total, int tid, SYNC &&sync) {
+__device__ __forceinline__ void end_of_step_ordered(Ctrl *ctrl, const StepConst &k, unsigned long long n, double ub, double mass,
+                                                    bool mass_step, unsigned index, unsigned total, int tid, SYNC &&sync) {
     __shared__ double gred[2][NTHREADS/32];
     __shared__ bool glast;
     const int lane = tid & 31, warp = tid >> 5;
+    const bool ordered = total <= (unsigned)MAX_PARTS;
+    double2 *parts = ctrl_parts(ctrl);
     ub = warp_sum(ub);
     if (mass_step) mass = warp_sum(mass);
     if (lane == 0) { gred[0][warp] = ub; gred[1][warp] = mass; }
@@ -276,20 +334,33 @@ __device__ __forceinline__ void end_of_step_group(Ctrl *ctrl, const StepConst &k
     if (tid == 0) {
         double s = 0.0, m = 0.0;
         for (int w = 0; w < NTHREADS/32; w++) { s += gred[0][w]; m += gred[1][w]; }
-        if (s != 0.0) atomicAdd(&ctrl->ub_slot[n & 1ULL], s);   // (also a NaN)
-        if (mass_step) atomicAdd(&ctrl->mass_slot[blockIdx.x & 255u], m);
+        if (ordered) __stcg(parts + index, make_double2(s, m));
+        else {
+            if (s != 0.0) atomicAdd(&ctrl->ub_slot[n & 1ULL], s);   // (also a NaN)
+            if (mass_step) atomicAdd(&ctrl->mass_slot[index & 255u], m);
+        }
         __threadfence();
         glast = atomicAdd(&ctrl->done, 1u) == total - 1u;
     }
     sync();
-    if (!glast || tid >= 32) return;
+    if (!glast) return;
     __threadfence();
-    double m = 0.0;
-    if (mass_step) {   // the 256 mass slots, summed by one warp
-        for (int i = lane; i < 256; i += 32) { m += __ldcg(&ctrl->mass_slot[i]); ctrl->mass_slot[i] = 0.0; }
-        m = warp_sum(m);
+    double s = 0.0, m = 0.0;
+    if (ordered) {
+        for (unsigned i = tid; i < total; i += NTHREADS) { const double2 p = __ldcg(parts + i); s += p.x; m += p.y; }
+        s = warp_sum(s);
+    } else if (mass_step) {
+        for (int i = tid; i < 256; i += NTHREADS) { m += __ldcg(&ctrl->mass_slot[i]); ctrl->mass_slot[i] = 0.0; }
     }
-    if (lane == 0) finish_step(ctrl, k, n, mass_step, m);
+    if (mass_step) m = warp_sum(m);
+    if (lane == 0) { gred[0][warp] = s; gred[1][warp] = m; }
+    sync();
+    if (tid == 0) {
+        s = 0.0; m = 0.0;
+        for (int w = 0; w < NTHREADS/32; w++) { s += gred[0][w]; m += gred[1][w]; }
+        if (ordered) ctrl->ub_slot[n & 1ULL] = s;
+        finish_step(ctrl, k, n, mass_step, m);
+    }
 }
 
 }  // namespace islbm

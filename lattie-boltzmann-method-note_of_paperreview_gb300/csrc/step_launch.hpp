@@ -16,6 +16,7 @@ struct StepLaunch {
     StepConst k;
     Ctrl *ctrl;                // device
     unsigned long long n;      // 1-based number of the step being computed
+    unsigned long long launch; // number of this step launch of the handle (1, 2, ...)
     bool les, macros_on, mass;
     void *macros[4];           // rho, u, v, w (compute type) when macros_on
     const void *tiled;         // TiledConst for the tiled kernel
@@ -23,6 +24,27 @@ struct StepLaunch {
     const void *chunk;         // ChunkConst for the chunk-marching kernel
     cudaStream_t stream;
 };
+
+// Programmatic dependent launch of consecutive step kernels: the next step's blocks may start, set up
+// their barriers and tensor memory and then wait for the previous step's end and its memory
+// (grid_dependency_wait) while that one's last blocks still run. A kernel launched this way reads and
+// writes nothing in global memory before the wait.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <class... P, class... A>
+cudaError_t launch_dependent(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t stream, A &&...args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 
 cudaError_t launch_step_gather(const StepLaunch &L);
 cudaError_t launch_step_tiled(const StepLaunch &L);

@@ -14,11 +14,10 @@ const RoleEntry &entry(int precision, int NX, bool les) {
     return t.e[les ? 1 : 0][NX == 32 ? 0 : NX == 64 ? 1 : NX == 128 ? 2 : 3];
 }
 
-// A segment costs about this many targets more than its targets: the 6 planes that fill the ring
-// before the first target, while the collide warps have nothing to do, and the pipeline's start
-// (from the busy times of SMs with one 84-target segment and with three of 24: 391 and 435
-// thousand cycles)
-constexpr double RAMP = 10.0;
+// A segment costs about this many targets more than its targets (the planes that fill the ring are
+// filtered faster than targets are collided): from the busy times of SMs with one segment of 84
+// targets and with two or three of 24 (407, 243 and 362 thousand cycles)
+constexpr double RAMP = 2.0;
 
 // Column split for `tiles` tiles on `slots` SMs, by the estimated makespan (a segment costs its targets
 // + RAMP): either every column in zsegs equal segments, taken round by round, or zmain long
@@ -48,7 +47,8 @@ void split_columns(int tiles, int slots, int NZ, TiledConst &tc) {
 bool roles_supported(const StepConst &k, int precision) {
     if (precision == ISLBM_FP64) return false;
     if (k.NX != 32 && k.NX != 64 && k.NX != 128 && k.NX != 256) return false;
-    return k.NY >= 512/k.NX + 6 && k.NZ >= 8;
+    // byte offsets into a population or field array are 32-bit in the kernel
+    return k.NY >= 512/k.NX + 6 && k.NZ >= 8 && (double)k.NX*k.NY*k.NZ*4.0 < 4294967296.0;
 }
 
 cudaError_t make_roles_const(const StepConst &k, int precision, bool les, const double *wx0, const double *wx2,
@@ -60,6 +60,7 @@ cudaError_t make_roles_const(const StepConst &k, int precision, bool les, const 
     split_columns(tiles, num_sms, k.NZ, tc);
     const long long items = (long long)tiles*(tc.zmain + tc.zsegs);
     tc.grid = tc.zmain ? num_sms : (int)std::min<long long>(items, num_sms);
+    tc.seats = tc.grid == num_sms;
     *out = tc;
     const RoleEntry &e = entry(precision, k.NX, les);
     out->smem_bytes = e.smem;

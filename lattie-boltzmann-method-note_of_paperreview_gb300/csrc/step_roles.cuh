@@ -8,7 +8,7 @@
 // plane waits for a CTA barrier: 42% of the issue slots were used. Here a CTA of 640 threads owns a
 // tile of 512 nodes (TY = 512/NX full rows), one CTA per SM, and four kinds of warps run at
 // their own pace, coupled by mbarriers only:
-//   * the front producer copies the planes of a wall-normal segment into two front stages
+//   * the front producer copies the planes of a wall-normal segment into the front stages
 //     (populations 3, 4, 7..10, 15..18 with three halo rows on each side; 5, 6, 11..14), the target
 //     producer the target planes' populations 0, 1, 2 and xi weights into target stages, each as 4D
 //     tensor-map boxes (tiles whose halo wraps around the period: row runs);
@@ -44,8 +44,10 @@ constexpr int COLLIDE_THREADS = 32*COLLIDE_WARPS;
 constexpr int FILTER_WARP0 = COLLIDE_WARPS, FRONT_WARP = FILTER_WARP0 + FILTER_WARPS, TARGET_WARP = FRONT_WARP + 1;
 constexpr int THREADS = 640;          // five warpgroups: collide, collide, row filter, quad filter, producers
 constexpr int ACTIVE_THREADS = 32*(TARGET_WARP + 1);
-// registers after the split: 2*144 + 2*80 + 32 = 480 = 5*96 that the CTA is launched with
-constexpr int REGS_COLLIDE = 144, REGS_FILTER = 80, REGS_PRODUCER = 32;
+// registers per thread of the warpgroups after the split: two collide groups, row filter, quad filter,
+// producers, together at most the 5*96 that the CTA is launched with
+template <class S> struct Regs { static constexpr int collide = 144, rows = 80, quads = 80, copies = 32; };   // 16-bit formats
+template <> struct Regs<float> { static constexpr int collide = 152, rows = 80, quads = 64, copies = 32; };
 constexpr int SLOTS = 8;              // ring planes
 
 // named barriers: 1 collide warps, 2 work item (batched kernel), 3, 4 filter row groups, 5 end of the
@@ -66,19 +68,6 @@ __device__ __forceinline__ unsigned long long global_ns() {
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
     return t;
 }
-// mbar_try_wait that may suspend the thread for up to 20 us
-__device__ __forceinline__ bool mbar_try_wait_for(uint64_t *bar, unsigned parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity), "r"(20000u)
-        : "memory");
-    return ok != 0;
-}
-
 // D3Q19 streamwise component of e_q (C/initialization.h:7-12 ordering)
 __host__ __device__ constexpr int ey_of(int q) {
     return (q == 3 || q == 7 || q == 8 || q == 15 || q == 17) ? 1 : (q == 4 || q == 9 || q == 10 || q == 16 || q == 18) ? -1 : 0;
@@ -89,7 +78,7 @@ __host__ __device__ constexpr int FQ(int i) {
 }
 
 // Shared-memory layout of one tile (compile-time offsets):
-//   two front stages; NTS target stages (populations 0, 1, 2 as TY rows, then the rows' duplicated
+//   NFS front stages; NTS target stages (populations 0, 1, 2 as TY rows, then the rows' duplicated
 //   xi weights, TY x 128 floats); ybuf [2][TY][2][NX/2] float4: streamwise-filtered (7, 8, 9, 10)
 //   by plane parity, the even and the odd node of each pair apart (consecutive threads, consecutive
 //   16 bytes); bfl [2][512] floats; mbarriers; timeout flag and TMEM address.
@@ -106,9 +95,15 @@ struct RLay {
     static constexpr int w_off = up128(3*plain_pop);
     static constexpr int target_bytes = w_off + TY*512;
     static constexpr unsigned target_tx = (unsigned)(3*plain_pop + TY*512);
-    static constexpr int NFS = 2;
     static constexpr int ybuf_bytes = 2*512*16, bfl_bytes = 2*512*4;
-    static constexpr int NTS = NFS*front_bytes + 4*target_bytes + ybuf_bytes + bfl_bytes + 1024 <= 227*1024 ? 4 : 2;
+    // front stages: as many as fit, up to three. The copies of a plane take about 2.5 us from issue to
+    // completion under load, longer than a plane's work: with two stages the copies' latency set
+    // the pace (FP32 256x128x192 without collisions and stores 184 us per step, with them 207)
+    static constexpr int room = 227*1024 - ybuf_bytes - bfl_bytes - 1536;
+    static constexpr int fit = (room - 2*target_bytes)/front_bytes;
+    static constexpr int NFS = fit > 3 ? 3 : fit;
+    static constexpr int NTS = NFS*front_bytes + 4*target_bytes <= room ? 4 : 2;
+    static_assert(NFS >= 2, "two front stages");
     static constexpr int target_off = NFS*front_bytes;
     static constexpr int ybuf_off = target_off + NTS*target_bytes;
     static constexpr int bfl_off = ybuf_off + ybuf_bytes;
@@ -131,6 +126,7 @@ template <class S, bool LES, int NXC>
 struct RoleKernel {
     using LY = RLay<S, NXC>;
     static constexpr int NX = NXC, PR = LY::PR, TY = LY::TY;
+    static_assert(2*Regs<S>::collide + Regs<S>::rows + Regs<S>::quads + Regs<S>::copies <= 480, "register split");
     struct Scal { float f6, f12, rho_mod, tau, lesC; };
     const S *__restrict__ fo;
     S *__restrict__ fn;
@@ -141,7 +137,14 @@ struct RoleKernel {
     Ctrl *ctrl;
     float *rho_out, *u_out, *v_out, *w_out;
     int macros_on, mass_on;
+    unsigned long long launch;   // number of this launch of the solve
 
+    // position in a ring of N stages: index and phase parity
+    template <int N> struct Stage {
+        int i = 0;
+        unsigned ph = 0;
+        __device__ __forceinline__ void next() { if (++i == N) { i = 0; ph ^= 1u; } }
+    };
     struct Piece {
         int y0, yskip, ta, tb, p0, p1;   // first row, rows done by the previous tile, targets, planes
     };
@@ -161,8 +164,8 @@ struct RoleKernel {
     // The work items of a CTA: M = zmain*tiles long segments, one for each of the first M CTAs, and
     // the rest of every column in zrest equal segments for the others (see split_columns)
     template <class F>
-    __device__ __forceinline__ void for_items(F &&f) const {
-        const int tiles = (k.NY + TY - 1)/TY, M = tc.zmain*tiles, b = (int)blockIdx.x;
+    __device__ __forceinline__ void for_items(int seat, F &&f) const {
+        const int tiles = (k.NY + TY - 1)/TY, M = tc.zmain*tiles, b = seat;
         if (b < M) {
             const int seg = b/tiles;
             f(make_piece(b - seg*tiles, seg*tc.zlen, (seg + 1)*tc.zlen));
@@ -175,18 +178,20 @@ struct RoleKernel {
         }
     }
 
-    // Wait for a phase of mbarrier b. The hardware suspends the thread (a poll loop with sleeps woke up
-    // late and took issue slots from the other roles). Bounded: after about two seconds, or
-    // once another thread of the CTA has given up, the thread stops waiting for good; the step then
-    // ends with ctrl->fault set.
+    // Wait for a phase of mbarrier b: no sleep between the tries (sleeping poll loops wake up late; FP32
+    // 217 instead of 207 us per step with them). Bounded: after about two seconds, or once another
+    // thread of the CTA has given up, the thread stops waiting for good; the step then ends with
+    // ctrl->fault set.
     __device__ __forceinline__ void wait(unsigned char *smem, int b, unsigned parity, bool &faulted) const {
         if (faulted) return;
         uint64_t *bar = (uint64_t *)(smem + LY::bar_off) + b;
-        if (mbar_try_wait_for(bar, parity)) return;
+        if (mbar_try_wait(bar, parity)) return;
         volatile int *flag = (volatile int *)(smem + LY::flag_off);
         const unsigned long long t0 = global_ns();
         do {
-            if (mbar_try_wait_for(bar, parity)) return;
+#pragma unroll 1
+            for (int i = 0; i < 64; i++)
+                if (mbar_try_wait(bar, parity)) return;
         } while (!*flag && global_ns() - t0 < 2000000000ULL);
         faulted = true;
         *flag = 1;
@@ -196,15 +201,15 @@ struct RoleKernel {
 
     // ---- producers (one lane each) ----
 
-    __device__ __forceinline__ void produce_front(unsigned char *smem, const Piece &P, unsigned &count, bool &faulted,
+    __device__ __forceinline__ void produce_front(unsigned char *smem, const Piece &P, Stage<LY::NFS> &at, unsigned &count, bool &faulted,
                                                   const CUtensorMap *tm) const {
         const int NY = k.NY;
         const size_t N = (size_t)NX*NY*k.NZ;
         constexpr int rows = TY + 6;
         const bool boxes = tm && P.y0 >= 3 && P.y0 + TY + 3 <= NY;
-        for (int p = P.p0; p <= P.p1; p++, count++) {
-            const int st = (int)(count % LY::NFS);
-            if (count >= LY::NFS) wait(smem, LY::B_FE + st, (count/LY::NFS - 1) & 1u, faulted);
+        for (int p = P.p0; p <= P.p1; p++, count++, at.next()) {
+            const int st = at.i;
+            wait(smem, LY::B_FE + st, at.ph ^ 1u, faulted);   // (at once in the first round)
             if (faulted || *(volatile int *)(smem + LY::flag_off)) return;   // no further copies after a timeout
             if (p == k.drill_plane) continue;                                // failure drill: this plane never arrives
             uint64_t *bar = bars(smem, LY::B_FF + st);
@@ -217,30 +222,36 @@ struct RoleKernel {
                 tma_load4(dst + LY::f_off(10), tm + 2, 0, P.y0, p, 5, bar);
                 tma_load4(dst + LY::f_off(12), tm + 3, 0, P.y0, p, 11, bar);
             } else {
+                // row runs: a halo that wraps around the period is two runs per population. Compile-time
+                // operands: a loop took 140 cycles per copy, and the wrapping tiles twice the others' time
                 const S *plane = fo + (size_t)p*NY*NX;
                 const int ys = P.y0 >= 3 ? P.y0 - 3 : P.y0 - 3 + NY;
-                const int first = min(rows, NY - ys);
-#pragma unroll 1
-                for (int i = 0; i < 10; i++) {
-                    unsigned char *d = dst + i*LY::halo_pop;
-                    const S *src = plane + (size_t)FQ(i)*N;
-                    bulk_g2s(d, src + (size_t)ys*NX, first*LY::row, bar);
-                    if (first < rows) bulk_g2s(d + first*LY::row, src, (rows - first)*LY::row, bar);
+                const unsigned first = (unsigned)min(rows, NY - ys)*LY::row, rest = (unsigned)LY::halo_pop - first;
+                const S *a = plane + (size_t)ys*NX;
+#pragma unroll
+                for (int i = 0; i < 10; i++) bulk_g2s(dst + i*LY::halo_pop, a + (size_t)FQ(i)*N, first, bar);
+                if (rest)
+#pragma unroll
+                    for (int i = 0; i < 10; i++) bulk_g2s(dst + i*LY::halo_pop + first, plane + (size_t)FQ(i)*N, rest, bar);
+                if (tm) {
+                    tma_load4(dst + LY::f_off(10), tm + 2, 0, P.y0, p, 5, bar);
+                    tma_load4(dst + LY::f_off(12), tm + 3, 0, P.y0, p, 11, bar);
+                } else {
+#pragma unroll
+                    for (int i = 10; i < 16; i++)
+                        bulk_g2s(dst + LY::f_off(i), plane + (size_t)FQ(i)*N + (size_t)P.y0*NX, LY::plain_pop, bar);
                 }
-#pragma unroll 1
-                for (int i = 10; i < 16; i++)
-                    bulk_g2s(dst + LY::f_off(i), plane + (size_t)FQ(i)*N + (size_t)P.y0*NX, LY::plain_pop, bar);
             }
         }
     }
 
-    __device__ __forceinline__ void produce_targets(unsigned char *smem, const Piece &P, unsigned &count, bool &faulted,
+    __device__ __forceinline__ void produce_targets(unsigned char *smem, const Piece &P, Stage<LY::NTS> &at, unsigned &count, bool &faulted,
                                                     const CUtensorMap *tm) const {
         const int NY = k.NY;
         const size_t N = (size_t)NX*NY*k.NZ;
-        for (int t = P.ta; t < P.tb; t++, count++) {
-            const int st = (int)(count % LY::NTS);
-            if (count >= LY::NTS) wait(smem, LY::B_TE + st, (count/LY::NTS - 1) & 1u, faulted);
+        for (int t = P.ta; t < P.tb; t++, count++, at.next()) {
+            const int st = at.i;
+            wait(smem, LY::B_TE + st, at.ph ^ 1u, faulted);
             if (faulted || *(volatile int *)(smem + LY::flag_off)) return;
             uint64_t *bar = bars(smem, LY::B_TF + st);
             unsigned char *dst = smem + LY::target_off + st*LY::target_bytes;
@@ -275,7 +286,6 @@ struct RoleKernel {
     // The streamwise sums of population FQ(q) for both rows from the eight halo rows
     template <int Q0, int NQ>
     __device__ __forceinline__ void y_filter(const S *base, V2 (&acc)[2][NQ]) const {
-#pragma unroll
         for (int q = 0; q < NQ; q++) acc[0][q] = acc[1][q] = V2(0.f);
 #pragma unroll
         for (int b = 0; b < 8; b++) {
@@ -290,25 +300,25 @@ struct RoleKernel {
     }
     // the ring slot is free once both collide warps of this lane quarter are done with its plane
     __device__ __forceinline__ void wait_slot(unsigned char *smem, unsigned seq, int w, bool &faulted) const {
-        if (seq >= SLOTS) wait(smem, LY::B_RE + w*SLOTS + (int)(seq % SLOTS), (seq/SLOTS - 1) & 1u, faulted);
+        wait(smem, LY::B_RE + w*SLOTS + (int)(seq % SLOTS), (seq/SLOTS & 1u) ^ 1u, faulted);
         tmem_fence_after();
     }
-    __device__ __forceinline__ void filtered(unsigned char *smem, unsigned seq, int w, int lane) const {
+    __device__ __forceinline__ void filtered(unsigned char *smem, int st, unsigned seq, int w, int lane) const {
         tmem_wait_st();
         tmem_fence_before();
         __syncwarp();
         if (lane == 0) {
-            mbar_arrive(bars(smem, LY::B_FE + (int)(seq % LY::NFS)));              // front stage read
+            mbar_arrive(bars(smem, LY::B_FE + st));                                // front stage read
             mbar_arrive(bars(smem, LY::B_RF + w*SLOTS + (int)(seq % SLOTS)));      // ring columns written
         }
     }
 
     // Row filter warps: y filter of 3, 4, 15..18, raw 5, 6 and x filter of 11..14
-    __device__ __forceinline__ void filter_rows(unsigned char *smem, unsigned seq, int w, int lane, uint32_t tl, bool &faulted) const {
+    __device__ __forceinline__ void filter_rows(unsigned char *smem, const Stage<LY::NFS> &at, unsigned seq, int w, int lane, uint32_t tl, bool &faulted) const {
         const int i = 32*w + lane, r0 = 2*(i/PR), j = i % PR, x0 = 2*j;
-        const unsigned char *front = smem + (int)(seq % LY::NFS)*LY::front_bytes;
+        const unsigned char *front = smem + at.i*LY::front_bytes;
         const uint32_t col = tl + 32u*(seq % SLOTS);
-        wait(smem, LY::B_FF + (int)(seq % LY::NFS), (seq/LY::NFS) & 1u, faulted);
+        wait(smem, LY::B_FF + at.i, at.ph, faulted);
         float o[2][8];
 #pragma unroll
         for (int r = 0; r < 2; r++)
@@ -331,16 +341,16 @@ struct RoleKernel {
             tmem_st16(col + 256u*r, v);
             tmem_st8(col + 256u*r + 24u, o[r][0], o[r][1], o[r][2], o[r][3], o[r][4], o[r][5], o[r][6], o[r][7]);
         }
-        filtered(smem, seq, w, lane);
+        filtered(smem, at.i, seq, w, lane);
     }
 
     // Quad filter warps: y and x filter of 7, 8, 9, 10, the y-filtered values of a node as one quad in ybuf
-    __device__ __forceinline__ void filter_quads(unsigned char *smem, unsigned seq, int w, int lane, uint32_t tl, bool &faulted) const {
+    __device__ __forceinline__ void filter_quads(unsigned char *smem, const Stage<LY::NFS> &at, unsigned seq, int w, int lane, uint32_t tl, bool &faulted) const {
         const int i = 32*w + lane, g = i/PR, r0 = 2*g, j = i % PR, x0 = 2*j;
-        const unsigned char *front = smem + (int)(seq % LY::NFS)*LY::front_bytes;
+        const unsigned char *front = smem + at.i*LY::front_bytes;
         float4 *yb = (float4 *)(smem + LY::ybuf_off) + (seq & 1u)*512 + r0*NX;   // [row][parity][pair]
         const uint32_t col = tl + 32u*(seq % SLOTS) + 16u;
-        wait(smem, LY::B_FF + (int)(seq % LY::NFS), (seq/LY::NFS) & 1u, faulted);
+        wait(smem, LY::B_FF + at.i, at.ph, faulted);
         {
             V2 acc[2][4];
             y_filter<2, 4>((const S *)front + r0*NX + x0, acc);
@@ -361,9 +371,11 @@ struct RoleKernel {
             float4 gv[8];
 #pragma unroll
             for (int a = 0; a < 8; a++) gv[a] = (a & 1) ? ev[(j - 1 + a/2) & (PR - 1)] : od[(j - 2 + a/2) & (PR - 1)];
-            V2 n0a = V2(0.f), n0b = n0a, n1a = n0a, n1b = n0a;   // (7, 8) and (9, 10) of node 0 / node 1
+            // (7, 8) and (9, 10) of node 0 / node 1
+            V2 n0a = V2(tc.wx[0])*V2(gv[0].x, gv[0].y), n0b = V2(tc.wx[0])*V2(gv[0].z, gv[0].w);
+            V2 n1a = V2(tc.wx[0])*V2(gv[1].x, gv[1].y), n1b = V2(tc.wx[0])*V2(gv[1].z, gv[1].w);
 #pragma unroll
-            for (int a = 0; a < 7; a++) {
+            for (int a = 1; a < 7; a++) {
                 const V2 wv = V2(tc.wx[a]);
                 n0a = wv*V2(gv[a].x, gv[a].y) + n0a;
                 n0b = wv*V2(gv[a].z, gv[a].w) + n0b;
@@ -377,11 +389,17 @@ struct RoleKernel {
 #pragma unroll
         for (int r = 0; r < 2; r++)
             tmem_st8(col + 256u*r, o[r][0], o[r][1], o[r][2], o[r][3], o[r][4], o[r][5], o[r][6], o[r][7]);
-        filtered(smem, seq, w, lane);
+        filtered(smem, at.i, seq, w, lane);
     }
-    __device__ __forceinline__ void filter_plane(unsigned char *smem, unsigned seq, int warp, int lane, uint32_t tl, bool &faulted) const {
-        if (warp < 4) filter_rows(smem, seq, warp, lane, tl, faulted);
-        else filter_quads(smem, seq, warp - 4, lane, tl, faulted);
+    __device__ __forceinline__ void filter_planes(unsigned char *smem, const Piece &P, Stage<LY::NFS> &at, unsigned &seq, int warp, int lane,
+                                                  uint32_t tl, bool &faulted) const {
+        const int planes = P.p1 - P.p0 + 1;
+        if (warp < 4)
+#pragma unroll 1
+            for (int i = 0; i < planes; i++, seq++, at.next()) filter_rows(smem, at, seq, warp, lane, tl, faulted);
+        else
+#pragma unroll 1
+            for (int i = 0; i < planes; i++, seq++, at.next()) filter_quads(smem, at, seq, warp - 4, lane, tl, faulted);
     }
 
     // Spanwise filter of one population (set 0: departure x - minSize, 1: x + minSize) for the node
@@ -410,10 +428,10 @@ struct RoleKernel {
     // xi combination of the seven ring planes seq .. seq + 6 with the duplicated-pair xi weights of
     // the target row w (7 x 16 floats: (xi3, xi3, xi4, xi4, xi5, xi5, xi6, xi6, xi15, xi15, ...,
     // xi18, xi18) per stencil point). Writes F[3..18].
-    __device__ __forceinline__ void xi_combine(uint32_t tl, unsigned seq, const float4 *w, V2 (&F)[19]) const {
+    // `under`: work done while the first two planes' loads are under way.
+    template <class U>
+    __device__ __forceinline__ void xi_combine(uint32_t tl, unsigned seq, const float4 *w, V2 (&F)[19], U &&under) const {
         V2 acc[16];
-#pragma unroll
-        for (int q = 0; q < 16; q++) acc[q] = V2(0.f);
         auto add = [&](const uint32_t (&g)[32], int c) {
             float4 wq[4];
 #pragma unroll
@@ -423,13 +441,18 @@ struct RoleKernel {
             // slot order 3, 4, 5, 6, 15, 16, 17, 18, 7, 8, 9, 10, 11, 12, 13, 14
             const V2 wj[16] = {x3, x4, x5, x6, x15, x16, x17, x18, x3, x3, x4, x4, x5, x5, x6, x6};
 #pragma unroll
-            for (int q = 0; q < 16; q++) acc[q] = wj[q]*V2(__uint_as_float(g[2*q]), __uint_as_float(g[2*q + 1])) + acc[q];
+            for (int q = 0; q < 16; q++) {
+                const V2 v(__uint_as_float(g[2*q]), __uint_as_float(g[2*q + 1]));
+                if (c == 0) acc[q] = wj[q]*v;
+                else acc[q] = wj[q]*v + acc[q];
+            }
         };
 #pragma unroll
         for (int c = 0; c < 7; c += 2) {
             uint32_t g0[32], g1[32];
             tmem_ld32(tl + 32u*((seq + c) % SLOTS), g0);
             if (c < 6) tmem_ld32(tl + 32u*((seq + c + 1) % SLOTS), g1);
+            if (c == 0) under();
             tmem_wait_ld();
             tmem_tie(g0);
             add(g0, c);
@@ -452,23 +475,33 @@ struct RoleKernel {
         else __syncwarp(PR == 32 ? 0xffffffffu : (0xffffu << (threadIdx.x & 16)));
     }
 
+    // a full value as the state holds it (the deviation formats: f - ref)
+    __device__ __forceinline__ static V2 stored(V2 v, int q) {
+        if constexpr (Storage<S>::dev) return v - V2((float)dev_ref(q));
+        else return v;
+    }
+    // half-way bounce-back: population q of a node from its opposite qs (deviations differ by the
+    // difference of their reference values)
+    __device__ __forceinline__ static V2 opposite(const S *node, size_t N, int qs, int q) { return stored(ld2g<S>(node + qs*N, qs), q); }
+
     // One flag type of the BFL rows (C/evolution.h:505-572) of a whole row y at plane z <= 1, called
     // by the row's threads together. dst / src: populations set and their opposites, the first without
     // and the other two with an x filter (n = 1 or 3); wall distance below one half: 7 x 7 (y, xi) sums
     // of the opposite populations per node, exchanged through `sums` for the x filter (a sum of
     // 7 x 7 x 7 terms per thread otherwise).
+    // Returns whether the row is set, with the populations as the state holds them in out.
     template <int N3>
-    __device__ __forceinline__ void bfl_type(V2 (&F)[19], int fl, const int (&dst)[N3], const int (&src)[N3], const int (&xset)[N3],
+    __device__ __forceinline__ bool bfl_type(V2 *out, int fl, const int (&dst)[N3], const int (&src)[N3], const int (&xset)[N3],
                                              int yset, int zset, int x0, int y, int z, int row, float *sums) const {
         const int NY = k.NY, nb = 2*k.NYD6, r = z*k.NYD6 + y + 3;
-        if (T.bfl_flag[fl*nb + r] != 1) return;
+        if (T.bfl_flag[fl*nb + r] != 1) return false;
         const size_t N = (size_t)NX*NY*k.NZ;
         const float q = T.bfl_q[fl*nb + r];
         if (q > 0.5f) {   // (1/(2Q)) f_opposite + ((2Q-1)/(2Q)) f at the node
             const S *nd = fo + ((size_t)z*NY + y)*NX + x0;
             const float c0 = 1.f/(2.f*q), c1 = (2.f*q - 1.f)/(2.f*q);
 #pragma unroll
-            for (int m = 0; m < N3; m++) F[dst[m]] = V2(c0)*ld2g<S>(nd + src[m]*N, src[m]) + V2(c1)*ld2g<S>(nd + dst[m]*N, dst[m]);
+            for (int m = 0; m < N3; m++) out[m] = stored(V2(c0)*ld2g<S>(nd + src[m]*N, src[m]) + V2(c1)*ld2g<S>(nd + dst[m]*N, dst[m]), dst[m]);
         }
         if (q < 0.5f) {
             const int iy = k.bfl_mode ? r : y + 3;   // reference: X weights at [i], Y weights at [j]
@@ -493,7 +526,7 @@ struct RoleKernel {
 #pragma unroll
                 for (int m = 0; m < N3; m++) g[m] = wz*in[m] + g[m];
             }
-            F[dst[0]] = g[0];
+            out[0] = stored(g[0], dst[0]);
             if constexpr (N3 == 3) {
                 float *s = sums + row*NX;   // [2][512]: two populations
                 row_sync(row);              // the row's previous sums have been read
@@ -510,89 +543,147 @@ struct RoleKernel {
 #pragma unroll
                         for (int a = 0; a < 7; a++) o[l] += bw(xset[m], a, ix)*s[(m - 1)*512 + ((x0 + l - 3 + a) & (NX - 1))];
                     }
-                    F[dst[m]] = V2(o[0], o[1]);
+                    out[m] = stored(V2(o[0], o[1]), dst[m]);
                 }
             }
+        }
+        return q > 0.5f || q < 0.5f;
+    }
+
+    // What the lower wall sets at planes z = 0 and 1 of a node pair: bounce-back (z = 0) and BFL rows. It
+    // depends on the old state only, so a piece that starts at the wall computes it before its first
+    // target, while the ring fills (after the ring it cost 2.6 us per plane, on the critical
+    // path of small grids). Indexed at run time: it lives in local memory.
+    struct Wall {
+        V2 v[2][8];        // 3, 7, 8 | 4, 9, 10 | 15 | 16
+        V2 bounce[5];      // 5, 11, 12, 15, 16 at z = 0
+        unsigned set[2];   // BFL types set at plane z
+    };
+    __device__ __forceinline__ void prepare_wall(Wall &w, int z0, int z1, int x0, int y, int row, float *sums) const {
+        const size_t N = (size_t)NX*k.NY*k.NZ;
+        if (z0 == 0) {
+            const S *b = fo + ((size_t)y*NX + x0);
+            w.bounce[0] = opposite(b, N, 6, 5);
+            w.bounce[1] = opposite(b, N, 14, 11);
+            w.bounce[2] = opposite(b, N, 13, 12);
+            w.bounce[3] = opposite(b, N, 18, 15);
+            w.bounce[4] = opposite(b, N, 17, 16);
+        }
+#pragma unroll 1
+        for (int z = z0; z < z1; z++) {
+            V2 *v = w.v[z];
+            unsigned m = bfl_type<3>(v, 0, {3, 7, 8}, {4, 10, 9}, {0, B_XB37, B_XB38}, B_YB378, B_XIB378, x0, y, z, row, sums) ? 1u : 0u;
+            m |= bfl_type<3>(v + 3, 1, {4, 9, 10}, {3, 8, 7}, {0, B_XB49, B_XB410}, B_YB4910, B_XIB4910, x0, y, z, row, sums) ? 2u : 0u;
+            m |= bfl_type<1>(v + 6, 2, {15}, {18}, {0}, B_YB15, B_XIB15, x0, y, z, row, sums) ? 4u : 0u;
+            m |= bfl_type<1>(v + 7, 3, {16}, {17}, {0}, B_YB16, B_XIB16, x0, y, z, row, sums) ? 8u : 0u;
+            w.set[z] = m;
         }
     }
 
     // Walls, BFL rows, collision and stores of the node pair (x0, x0 + 1) at row y, plane z, whose
-    // streamed populations are in F (filtered values, deviations for the deviation formats)
-    __device__ __forceinline__ void finish(V2 (&F)[19], int x0, int y, int row, int z, const Scal &sc, float &ub, V2 &mass, float *sums) const {
+    // streamed populations are in F as the state holds them (deviations for the deviation formats)
+    // (WALL: z <= 1, the planes that the lower wall sets)
+    template <bool WALL>
+    __device__ __forceinline__ void finish(V2 (&F)[19], int x0, int y, int z, const Scal &sc, float &ub, V2 &mass, const Wall *wall) const {
         const int NY = k.NY;
         const size_t N = (size_t)NX*NY*k.NZ;
-        const unsigned node = (unsigned)(((size_t)z*NY + y)*NX + x0);
-        if constexpr (Storage<S>::dev) {
-#pragma unroll
-            for (int q = 0; q < 19; q++) F[q] = F[q] + V2((float)dev_ref(q));
-        }
-        const S *b = fo + node;
-        if (z <= 1) {
-            if (z == 0) {
-                F[5] = ld2g<S>(b + 6*N, 6); F[11] = ld2g<S>(b + 14*N, 14); F[12] = ld2g<S>(b + 13*N, 13);
-                F[15] = ld2g<S>(b + 18*N, 18); F[16] = ld2g<S>(b + 17*N, 17);
-            }
-            bfl_type<3>(F, 0, {3, 7, 8}, {4, 10, 9}, {0, B_XB37, B_XB38}, B_YB378, B_XIB378, x0, y, z, row, sums);
-            bfl_type<3>(F, 1, {4, 9, 10}, {3, 8, 7}, {0, B_XB49, B_XB410}, B_YB4910, B_XIB4910, x0, y, z, row, sums);
-            bfl_type<1>(F, 2, {15}, {18}, {0}, B_YB15, B_XIB15, x0, y, z, row, sums);
-            bfl_type<1>(F, 3, {16}, {17}, {0}, B_YB16, B_XIB16, x0, y, z, row, sums);
+        // byte offsets fit 32 bits (roles_supported): a uniform base and a 32-bit offset per store
+        // instead of a 64-bit address each (FP16 193 -> 182 us per step on 256x128x192)
+        const unsigned node = (unsigned)((z*NY + y)*NX + x0), off = node*(unsigned)sizeof(S), moff = node*4u;
+        const S *b = (const S *)((const char *)fo + off);
+        if constexpr (WALL) {
+            if (z == 0) { F[5] = wall->bounce[0]; F[11] = wall->bounce[1]; F[12] = wall->bounce[2]; F[15] = wall->bounce[3]; F[16] = wall->bounce[4]; }
+            const V2 *v = wall->v[z];
+            const unsigned m = wall->set[z];
+            if (m & 1u) { F[3] = v[0]; F[7] = v[1]; F[8] = v[2]; }
+            if (m & 2u) { F[4] = v[3]; F[9] = v[4]; F[10] = v[5]; }
+            if (m & 4u) F[15] = v[6];
+            if (m & 8u) F[16] = v[7];
         }
         if (z == k.NZ - 1) {
-            F[6] = ld2g<S>(b + 5*N, 5); F[13] = ld2g<S>(b + 12*N, 12); F[14] = ld2g<S>(b + 11*N, 11);
-            F[17] = ld2g<S>(b + 16*N, 16); F[18] = ld2g<S>(b + 15*N, 15);
+            F[6] = opposite(b, N, 5, 6); F[13] = opposite(b, N, 12, 13); F[14] = opposite(b, N, 11, 14);
+            F[17] = opposite(b, N, 16, 17); F[18] = opposite(b, N, 15, 18);
         }
         V2 rho, u1, v1, w1;
-        collide<LES>(F, sc.rho_mod, sc.f6, sc.f12, sc.tau, sc.lesC, rho, u1, v1, w1);
+        if constexpr (Storage<S>::dev) collide<LES, true>(F, sc.rho_mod, sc.f6, sc.f12, sc.tau, sc.lesC, rho, u1, v1, w1);
+        else collide_x2<LES>(F, sc.rho_mod, sc.f6, sc.f12, sc.tau, sc.lesC, rho, u1, v1, w1);
 #pragma unroll
-        for (int q = 0; q < 19; q++) st2<S>(fnq[q] + node, F[q], q);
+        for (int q = 0; q < 19; q++) st2s<S>((S *)((char *)fnq[q] + off), F[q]);
         if (macros_on) {
-            *(float2 *)(rho_out + node) = rho.v; *(float2 *)(u_out + node) = u1.v;
-            *(float2 *)(v_out + node) = v1.v; *(float2 *)(w_out + node) = w1.v;
+            *(float2 *)((char *)rho_out + moff) = rho.v; *(float2 *)((char *)u_out + moff) = u1.v;
+            *(float2 *)((char *)v_out + moff) = v1.v; *(float2 *)((char *)w_out + moff) = w1.v;
         }
         // column partials in FP32 (at most NZ terms), folded into FP64 once per piece
         if (y == k.yplane) ub += (v1.v.x*T.dxf[x0] + v1.v.y*T.dxf[x0 + 1])*T.dzf[z];
         mass = mass + rho;   // a non-finite density makes the mass sum non-finite (checked once per piece)
     }
 
-    // All targets of a piece for collide warp `warp` (lane quarter warp % 4, row of the pair warp / 4);
-    // seq0: ring sequence number of plane p0, tcount: target stages used before this piece
-    __device__ __forceinline__ void collide_piece(unsigned char *smem, const Piece &P, unsigned seq0, unsigned tcount, int warp, int lane,
-                                                  uint32_t tl, const Scal &sc, float &ub, V2 &mass, bool &faulted) const {
-        const int w = warp & 3, i = 32*w + lane, row = 2*(i/PR) + (warp >> 2), x0 = 2*(i % PR), y = P.y0 + row;
-        float *sums = (float *)(smem + LY::bfl_off);
-        const bool own = row >= P.yskip;
-        int freed = P.p0;
+    // A collide warp's node pair and its place in the pipelines
+    struct Pair {
+        int w, i, row, x0, y;      // lane quarter, pair in the tile, row and columns
+        int freed;                 // first ring plane not yet released
+        unsigned seq0, tcount;     // ring sequence number of plane p0, target stages used
+        uint32_t tl;
+        bool own;                  // false: the previous tile's row
+    };
+    // Targets t0 .. t1 - 1 of a piece
+    template <bool WALL>
+    __device__ __forceinline__ void collide_targets(unsigned char *smem, const Piece &P, int t0, int t1, Pair &L, int lane, const Scal &sc,
+                                                    float &ub, V2 &mass, bool &faulted, const Wall *wall) const {
 #pragma unroll 1
-        for (int t = P.ta; t < P.tb; t++, tcount++) {
-            const int st = (int)(tcount % LY::NTS), base = window_base(t);
+        for (int t = t0; t < t1; t++, L.tcount++) {
+            const int st = (int)(L.tcount % LY::NTS), base = window_base(t);
             const unsigned char *stage = smem + LY::target_off + st*LY::target_bytes;
             V2 F[19];
             __syncwarp();   // (rows of one warp may have parted at the walls, the ring loads are warp-wide)
-            wait(smem, LY::B_TF + st, (tcount/LY::NTS) & 1u, faulted);
-            {
-                const S *q0 = (const S *)stage + row*NX;
+            wait(smem, LY::B_TF + st, (L.tcount/LY::NTS) & 1u, faulted);
+            const unsigned seq = L.seq0 + (unsigned)(base - P.p0), last = seq + 6;
+            wait(smem, LY::B_RF + L.w*SLOTS + (int)(last % SLOTS), (last/SLOTS) & 1u, faulted);
+            tmem_fence_after();
+            xi_combine(L.tl, seq, (const float4 *)(stage + LY::w_off) + L.row*32, F, [&] {
+                const S *q0 = (const S *)stage + L.row*NX;
                 float o[4];
-                F[0] = ld2v<S>(q0 + x0);
-                x_filter(q0 + TY*NX, i % PR, 0, o[0], o[1]);
-                x_filter(q0 + 2*TY*NX, i % PR, 1, o[2], o[3]);
+                F[0] = ld2v<S>(q0 + L.x0);
+                x_filter(q0 + TY*NX, L.i % PR, 0, o[0], o[1]);
+                x_filter(q0 + 2*TY*NX, L.i % PR, 1, o[2], o[3]);
                 F[1] = V2(o[0], o[1]);
                 F[2] = V2(o[2], o[3]);
-            }
-            const unsigned seq = seq0 + (unsigned)(base - P.p0), last = seq + 6;
-            wait(smem, LY::B_RF + w*SLOTS + (int)(last % SLOTS), (last/SLOTS) & 1u, faulted);
-            tmem_fence_after();
-            xi_combine(tl, seq, (const float4 *)(stage + LY::w_off) + row*32, F);
+            });
             tmem_fence_before();
             __syncwarp();
             // planes below the next target's window are free; so is the target stage
             const int next = t + 1 < P.tb ? window_base(t + 1) : P.p1 + 1;
             if (lane == 0) {
                 mbar_arrive(bars(smem, LY::B_TE + st));
-                for (int p = freed; p < next; p++) mbar_arrive(bars(smem, LY::B_RE + w*SLOTS + (int)((seq0 + (unsigned)(p - P.p0)) % SLOTS)));
+                for (int p = L.freed; p < next; p++)
+                    mbar_arrive(bars(smem, LY::B_RE + L.w*SLOTS + (int)((L.seq0 + (unsigned)(p - P.p0)) % SLOTS)));
             }
-            freed = next;
-            if (own) finish(F, x0, y, row, t, sc, ub, mass, sums);
+            L.freed = next;
+            if (L.own) finish<WALL>(F, L.x0, L.y, t, sc, ub, mass, wall);
         }
+    }
+    // All targets of a piece for collide warp `warp` (lane quarter warp % 4, row of the pair warp / 4);
+    // seq0: ring sequence number of plane p0, tcount: target stages used before this piece. The wall
+    // planes run in a loop of their own, so that the main one carries none of their state.
+    __device__ __forceinline__ void collide_piece(unsigned char *smem, const Piece &P, unsigned seq0, unsigned tcount, int warp, int lane,
+                                                  uint32_t tl, const Scal &sc, float &ub, V2 &mass, bool &faulted) const {
+        Pair L;
+        L.w = warp & 3;
+        L.i = 32*L.w + lane;
+        L.row = 2*(L.i/PR) + (warp >> 2);
+        L.x0 = 2*(L.i % PR);
+        L.y = P.y0 + L.row;
+        L.freed = P.p0;
+        L.seq0 = seq0;
+        L.tcount = tcount;
+        L.tl = tl;
+        L.own = L.row >= P.yskip;
+        if (P.ta <= 1) {
+            Wall wall;
+            if (L.own) prepare_wall(wall, P.ta, min(P.tb, 2), L.x0, L.y, L.row, (float *)(smem + LY::bfl_off));
+            collide_targets<true>(smem, P, P.ta, min(P.tb, 2), L, lane, sc, ub, mass, faulted, &wall);
+        }
+        collide_targets<false>(smem, P, max(P.ta, 2), P.tb, L, lane, sc, ub, mass, faulted, nullptr);
     }
 
     // ---- CTA set-up and end ----
@@ -625,6 +716,25 @@ struct RoleKernel {
         __syncthreads();
         tmem_fence_after();
     }
+    // The CTA's place in the work list, by the SM it runs on: neighbouring tiles on neighbouring SMs share
+    // the halo rows they read at the same time (256x128x192, without dependent launches: FP32 181
+    // -> 178, FP16 181 -> 171 us per step; with an arbitrary placement 230 and 275, and dependent
+    // launches place CTAs as SMs become free). Any placement is valid: a CTA takes the seat of its
+    // SM or the next free one; a seat is free to a launch that no earlier or equal number holds.
+    // (Grids smaller than the GPU go by block number.) The claim runs beside the CTA's set-up.
+    __device__ __forceinline__ void claim_seat(unsigned char *smem, int tid) const {
+        if (tid != 32) return;   // not the warp that allocates tensor memory
+        const unsigned n = gridDim.x;
+        unsigned s = blockIdx.x;
+        if (tc.seats && n <= (unsigned)MAX_SEATS) {
+            unsigned sm;
+            asm volatile("mov.u32 %0, %smid;" : "=r"(sm));
+            unsigned long long *seats = ctrl_seats(ctrl);
+            s = sm < n ? sm : n - 1;
+            for (unsigned i = 1; i < n && atomicMax(seats + s, launch) >= launch; i++) s = s + 1 == n ? 0 : s + 1;
+        }
+        *(volatile int *)(smem + LY::flag_off + 4) = (int)s;
+    }
     __device__ static uint32_t tmem_base(unsigned char *smem) { return *(volatile uint32_t *)(smem + LY::flag_off + 8); }
     // by the collide warps, after their last use of the ring; the filter warps arrive after their last
     // store (ring_done), so that none is under way even after a timed-out pipeline
@@ -645,15 +755,18 @@ struct RoleKernel {
     __device__ __forceinline__ void run(unsigned char *smem, const CUtensorMap *tm) const {
         const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
         if (smem_u32(smem) & 127u) tm = nullptr;   // tensor copies need 128-byte aligned destinations
+        claim_seat(smem, tid);
         init(smem, tid);
+        const int seat = *(volatile int *)(smem + LY::flag_off + 4);
+        grid_dependency_wait();   // nothing above touches global memory but the seats
         bool faulted = false;
         if (warp < COLLIDE_WARPS) {
-            regs_inc<REGS_COLLIDE>();
+            regs_inc<Regs<S>::collide>();
             const uint32_t tl = tmem_base(smem) + ((uint32_t)(32*(warp & 3)) << 16) + 256u*(uint32_t)(warp >> 2);
             double ub_total = 0.0, mass_total = 0.0;
             const Scal sc = scalars();
             unsigned seq = 0, tcount = 0;
-            for_items([&](const Piece &P) {
+            for_items(seat, [&](const Piece &P) {
                 float ub = 0.f;
                 V2 mass = V2(0.f);
                 collide_piece(smem, P, seq, tcount, warp, lane, tl, sc, ub, mass, faulted);
@@ -664,27 +777,31 @@ struct RoleKernel {
                 ub_total += (double)ub;
                 mass_total += (double)m;
             });
+            // the next step's CTAs may come now: triggered at the start, they took SMs one by one as
+            // these became free, which scatters neighbouring tiles
+            grid_dependency_trigger();
             ring_free(smem, tid);
-            end_of_step_group<COLLIDE_THREADS>(ctrl, k, tc.n, ub_total, mass_total, mass_on != 0, gridDim.x, tid,
-                                               [] { bar_sync(BAR_COLLIDE, COLLIDE_THREADS); });
+            end_of_step_ordered<COLLIDE_THREADS>(ctrl, k, tc.n, ub_total, mass_total, mass_on != 0, (unsigned)seat, gridDim.x, tid,
+                                                 [] { bar_sync(BAR_COLLIDE, COLLIDE_THREADS); });
         } else if (warp < FRONT_WARP) {
-            regs_dec<REGS_FILTER>();
+            if (warp < FILTER_WARP0 + 4) regs_dec<Regs<S>::rows>();
+            else regs_dec<Regs<S>::quads>();
             const int w = warp - FILTER_WARP0;
             const uint32_t tl = tmem_base(smem) + ((uint32_t)(32*(w & 3)) << 16);
             unsigned seq = 0;
-            for_items([&](const Piece &P) {
-#pragma unroll 1
-                for (int p = P.p0; p <= P.p1; p++, seq++) filter_plane(smem, seq, w, lane, tl, faulted);
-            });
+            Stage<LY::NFS> at;
+            for_items(seat, [&](const Piece &P) { filter_planes(smem, P, at, seq, w, lane, tl, faulted); });
             ring_done();
         } else {
-            regs_dec<REGS_PRODUCER>();
+            regs_dec<Regs<S>::copies>();
             unsigned count = 0;
             if (warp == FRONT_WARP && lane == 0) {
-                for_items([&](const Piece &P) { produce_front(smem, P, count, faulted, tm); });
+                Stage<LY::NFS> at;
+                for_items(seat, [&](const Piece &P) { produce_front(smem, P, at, count, faulted, tm); });
                 drain(smem, LY::B_FF, LY::NFS, count);
             } else if (warp == TARGET_WARP && lane == 0) {
-                for_items([&](const Piece &P) { produce_targets(smem, P, count, faulted, tm); });
+                Stage<LY::NTS> at;
+                for_items(seat, [&](const Piece &P) { produce_targets(smem, P, at, count, faulted, tm); });
                 drain(smem, LY::B_TF, LY::NTS, count);
             }
         }
@@ -721,6 +838,7 @@ step_roles_batch_kernel(const RoleBatchDesc<S, LES, NXC> *__restrict__ descs, co
     KT &K = *(KT *)kbuf;
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     KT::init(smem, tid);
+    grid_dependency_wait();
     bool faulted = false;
     // the descriptor of item `it` into K, by the 14 active warps together
     auto load_item = [&](int it, int2 &w, const CUtensorMap *&tm) {
@@ -748,7 +866,7 @@ step_roles_batch_kernel(const RoleBatchDesc<S, LES, NXC> *__restrict__ descs, co
     int2 w;
     const CUtensorMap *tm;
     if (warp < COLLIDE_WARPS) {
-        regs_inc<REGS_COLLIDE>();
+        regs_inc<Regs<S>::collide>();
         const uint32_t tl = KT::tmem_base(smem) + ((uint32_t)(32*(warp & 3)) << 16) + 256u*(uint32_t)(warp >> 2);
         unsigned seq = 0, tcount = 0;
         for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
@@ -761,30 +879,34 @@ step_roles_batch_kernel(const RoleBatchDesc<S, LES, NXC> *__restrict__ descs, co
             tcount += (unsigned)(P.tb - P.ta);
             const float m = mass.v.x + mass.v.y;
             if (!isfinite(m)) K.ctrl->nonfinite = 1u;
-            end_of_step_group<COLLIDE_THREADS>(K.ctrl, K.k, K.tc.n, (double)ub, (double)m, K.mass_on != 0,
-                                               (unsigned)(descs[w.x].ntiles*descs[w.x].nseg), tid,
-                                               [] { bar_sync(BAR_COLLIDE, COLLIDE_THREADS); });
+            end_of_step_ordered<COLLIDE_THREADS>(K.ctrl, K.k, K.tc.n, (double)ub, (double)m, K.mass_on != 0, (unsigned)w.y,
+                                                 (unsigned)(descs[w.x].ntiles*descs[w.x].nseg), tid,
+                                                 [] { bar_sync(BAR_COLLIDE, COLLIDE_THREADS); });
         }
+        grid_dependency_trigger();
         KT::ring_free(smem, tid);
     } else if (warp < FRONT_WARP) {
-        regs_dec<REGS_FILTER>();
+        if (warp < FILTER_WARP0 + 4) regs_dec<Regs<S>::rows>();
+        else regs_dec<Regs<S>::quads>();
         const uint32_t tl = KT::tmem_base(smem) + ((uint32_t)(32*(warp & 3)) << 16);
         unsigned seq = 0;
+        typename KT::template Stage<KT::LY::NFS> at;
         for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
             const typename KT::Piece P = load_item(it, w, tm);
-#pragma unroll 1
-            for (int p = P.p0; p <= P.p1; p++, seq++) K.filter_plane(smem, seq, warp - FILTER_WARP0, lane, tl, faulted);
+            K.filter_planes(smem, P, at, seq, warp - FILTER_WARP0, lane, tl, faulted);
         }
         KT::ring_done();
     } else {
-        regs_dec<REGS_PRODUCER>();
+        regs_dec<Regs<S>::copies>();
         if (warp > TARGET_WARP) return;
         unsigned count = 0;
+        typename KT::template Stage<KT::LY::NFS> fat;
+        typename KT::template Stage<KT::LY::NTS> tat;
         for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
             const typename KT::Piece P = load_item(it, w, tm);
             if (lane == 0) {
-                if (warp == FRONT_WARP) K.produce_front(smem, P, count, faulted, tm);
-                else K.produce_targets(smem, P, count, faulted, tm);
+                if (warp == FRONT_WARP) K.produce_front(smem, P, fat, count, faulted, tm);
+                else K.produce_targets(smem, P, tat, count, faulted, tm);
             }
             __syncwarp();
         }
@@ -814,11 +936,11 @@ struct RoleOps {
         K.rho_out = (float *)L.macros[0]; K.u_out = (float *)L.macros[1];
         K.v_out = (float *)L.macros[2]; K.w_out = (float *)L.macros[3];
         K.macros_on = L.macros_on; K.mass_on = L.mass;
+        K.launch = L.launch;
         RoleTM T;
         std::memset((void *)&T, 0, sizeof(T));
         if (L.pmaps) std::memcpy((void *)T.m, L.pmaps, sizeof(T.m));
-        step_roles_kernel<S, LES, NXC><<<K.tc.grid, THREADS, smem, L.stream>>>(K, T, L.pmaps != nullptr);
-        return cudaGetLastError();
+        return launch_dependent(step_roles_kernel<S, LES, NXC>, K.tc.grid, THREADS, smem, L.stream, K, T, (int)(L.pmaps != nullptr));
     }
     static size_t desc_bytes() { return sizeof(D); }
     static void fill(const Tables<float> &T, const StepConst &k, const TiledConst &tc, Ctrl *ctrl, void *const macros[4],
@@ -836,8 +958,7 @@ struct RoleOps {
         std::memcpy(out, (const void *)&d, sizeof(d));
     }
     static cudaError_t launch_batch(const void *descs, const int2 *items, int nitems, int grid, int macros_on, cudaStream_t st) {
-        step_roles_batch_kernel<S, LES, NXC><<<grid, THREADS, smem, st>>>((const D *)descs, items, nitems, macros_on);
-        return cudaGetLastError();
+        return launch_dependent(step_roles_batch_kernel<S, LES, NXC>, grid, THREADS, smem, st, (const D *)descs, items, nitems, macros_on);
     }
     // on the current device; every solve does this at its set-up, before any launch or capture
     static cudaError_t prepare() {

@@ -227,7 +227,7 @@ struct TiledKernel {
 #pragma unroll
         for (int q = 0; q < 19; q++) Fl[q] = F[q];
         float rho_s, u1, v1, w1;
-        collide<LES>(Fl, sc.rho_mod, sc.f6, sc.f12, sc.tau, sc.lesC, rho_s, u1, v1, w1);
+        collide_pairs<float, LES>(Fl, sc.rho_mod, sc.f6, sc.f12, sc.tau, sc.lesC, rho_s, u1, v1, w1);
 #pragma unroll
         for (int q = 0; q < 19; q++) store_f<S>(fnq[q], (unsigned)node, q, Fl[q]);
         if (macros_on) { rho_out[node] = rho_s; u_out[node] = u1; v_out[node] = v1; w_out[node] = w1; }

@@ -27,6 +27,7 @@ struct TiledConst {
     // role-specialised kernel (step_roles.cu): zmain segments of zlen targets from the bottom of every
     // column, the rest of the column in zsegs equal ones
     int zmain, zlen;
+    int seats;                    // one CTA per SM: blocks take their work by SM (claim_seat)
     unsigned long long n;         // step number (set per launch)
 };
 

@@ -341,6 +341,11 @@ int copy_macro(islbm_handle *h, int which, double *out, int layout) {
         CK(cudaStreamSynchronize(h->stream));
         return ISLBM_OK;
     }
+    if (layout == ISLBM_LAYOUT_UNIQUE) {   // FP64 fields: as they are
+        CK(cudaMemcpyAsync(out, h->macros[which], N*8, cudaMemcpyDeviceToHost, h->stream));
+        CK(cudaStreamSynchronize(h->stream));
+        return ISLBM_OK;
+    }
     std::vector<double> tmp(N);
     if (h->celem == 8) {
         CK(cudaMemcpyAsync(tmp.data(), h->macros[which], N*8, cudaMemcpyDeviceToHost, h->stream));
@@ -351,8 +356,7 @@ int copy_macro(islbm_handle *h, int which, double *out, int layout) {
         CK(cudaStreamSynchronize(h->stream));
         for (size_t i = 0; i < N; i++) tmp[i] = f[i];
     }
-    if (layout == ISLBM_LAYOUT_REFERENCE) unique_to_reference(h, tmp.data(), out);
-    else std::memcpy(out, tmp.data(), N*8);
+    unique_to_reference(h, tmp.data(), out);
     return ISLBM_OK;
 }
 
@@ -476,6 +480,7 @@ namespace islbm {
 int handle_init(const islbm_params *p, islbm_handle *h) { return init_impl(p, h); }
 void handle_free(islbm_handle *h) { free_handle_impl(h); }
 int report_cuda(cudaError_t e, const char *what) { return cuda_fail(e, what); }
+cudaError_t handle_xfer(islbm_handle *h) { return xfer_buffer(h); }
 void unique_to_reference_layout(const islbm_handle *h, const double *u, double *r) { unique_to_reference(h, u, r); }
 void reference_to_unique_layout(const islbm_handle *h, const double *r, double *u) { reference_to_unique(h, r, u); }
 int report_status(int status, const char *msg) {

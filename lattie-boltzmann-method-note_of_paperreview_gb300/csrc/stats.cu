@@ -39,6 +39,11 @@ __global__ void stats_kernel(const C *__restrict__ rho, const C *__restrict__ u,
     }
 }
 
+// time mean of one quantity: sum / samples
+__global__ void mean_kernel(const double *__restrict__ sum, double *__restrict__ out, size_t n, double inv) {
+    for (size_t i = blockIdx.x*(size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x*blockDim.x) out[i] = __dmul_rn(sum[i], inv);
+}
+
 // Squared velocity gradients of MeanVars' companion (MeanDerivatives, C/statistics.h:176-222):
 // x and y by the fourth-order central difference (8 (f[+1] - f[-1]) - (f[+2] - f[-2])) / 12 / h,
 // periodic; z by five weights per node over the nodes n .. n + 4 of its column,
@@ -191,15 +196,27 @@ int islbm_stats_mean(islbm_handle *h, int quantity, double *out, int layout) {
     if (!h->stats || h->stats_samples == 0) return report_status(ISLBM_ERR_NOT_SUPPORTED, "no statistics samples");
     cudaError_t e = cudaSetDevice(h->device);
     if (e != cudaSuccess) return report_cuda(e, "cudaSetDevice");
-    std::vector<double> sum(h->N);
-    e = cudaMemcpyAsync(sum.data(), h->stats + (size_t)quantity*h->N, h->N*sizeof(double), cudaMemcpyDeviceToHost,
-                        h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    if (e != cudaSuccess) return report_cuda(e, "statistics read");
+    // scaled on the device and copied straight into the caller's buffer (unique layout): the detour
+    // through a host vector took 0.70 ms per quantity of 128x64x96, four fifths of a window's read
     const double inv = 1.0/(double)h->stats_samples;
-    for (size_t i = 0; i < h->N; i++) sum[i] *= inv;
-    if (layout == ISLBM_LAYOUT_REFERENCE) unique_to_reference_layout(h, sum.data(), out);
-    else std::memcpy(out, sum.data(), h->N*sizeof(double));
+    std::vector<double> mean(layout == ISLBM_LAYOUT_REFERENCE ? h->N : 0);
+    double *dst = mean.empty() ? out : mean.data();
+    e = handle_xfer(h);
+    if (e == cudaErrorMemoryAllocation) {   // no device memory for the buffer: scaled on the host
+        (void)cudaGetLastError();
+        e = cudaMemcpyAsync(dst, h->stats + (size_t)quantity*h->N, h->N*sizeof(double), cudaMemcpyDeviceToHost, h->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+        if (e == cudaSuccess)
+            for (size_t i = 0; i < h->N; i++) dst[i] *= inv;
+    } else if (e == cudaSuccess) {
+        const unsigned grid = (unsigned)std::min<size_t>(4096, (h->N + 255)/256);
+        mean_kernel<<<grid, 256, 0, h->stream>>>(h->stats + (size_t)quantity*h->N, h->xfer, h->N, inv);
+        e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaMemcpyAsync(dst, h->xfer, h->N*sizeof(double), cudaMemcpyDeviceToHost, h->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    }
+    if (e != cudaSuccess) return report_cuda(e, "statistics read");
+    if (layout == ISLBM_LAYOUT_REFERENCE) unique_to_reference_layout(h, mean.data(), out);
     return ISLBM_OK;
 }
 

@@ -466,7 +466,7 @@ int init_impl(const islbm_params *pp, islbm_handle *h) {
         }
         if (p.kernel != ISLBM_KERNEL_AUTO && !h->use_tiled) { g_last = "tiled kernel does not support this grid"; return ISLBM_ERR_NOT_SUPPORTED; }
     }
-    if (p.kernel == ISLBM_KERNEL_AUTO && !h->use_tiled) {
+    if (p.kernel == ISLBM_KERNEL_AUTO && !h->use_tiled && chunk_supported(k, p.precision)) {
         CK(make_chunk_const(k, p.precision, p.les_cs > 0.0, wx0, wx2, wy0, wy2, sms, &h->chunk));
         h->chunked = true;
     }

@@ -1,6 +1,6 @@
-// Chunk-marching step kernel: the separable interpolation on any grid and storage format.
+// Chunk-marching step kernel: the separable interpolation on any grid in FP64 and FP32.
 //
-// Same step as stream_collide (C/evolution.h:358-684). It serves FP64 (the parity precision) and
+// Same step as stream_collide (C/evolution.h:358-684). It serves FP64 (the parity precision) and FP32 on
 // every grid without a tiled layout (spanwise widths other than the tiled ones, streamwise counts
 // that are no multiple of a tile's rows), where the gather kernel evaluates each departure point's
 // 7 x 7 x 7 stencil by itself: about 2,500 multiply-adds and adds per node. Here the streamwise and
@@ -54,8 +54,8 @@ __device__ __forceinline__ int wrap_any(int v, int n) {
 template <class S, bool LES>
 struct Chunk {
     using C = typename Storage<S>::C;
-    const S *__restrict__ fo;
-    S *__restrict__ fn;
+    const S *fq[19];           // old populations, one array each: uniform bases for 32-bit byte offsets
+    S *fnq[19];
     Tables<C> T;
     StepConst k;
     ChunkConst cc;
@@ -65,8 +65,11 @@ struct Chunk {
     C ux0[7], ux2[7], uy0[7], uy2[7];   // FP32: uniform spacing, the weights of the first node
     int macros_on, mass_on;
 
-    __device__ __forceinline__ C val(const S *p) const { return to_c(__ldg(p)); }   // stored value (a deviation for FP16 / BF16)
-    __device__ __forceinline__ C full(const S *p, C r) const { if constexpr (Storage<S>::dev) return val(p) + r; else return val(p); }
+    // stored value (a deviation for FP16 / BF16) of population q at a byte offset (chunk_supported: 32 bits).
+    // 64-bit addresses, one per load, were 40% of the kernel's instructions (FP32 187x91x131 224 us per step).
+    __device__ __forceinline__ C val(int q, unsigned off) const { return to_c(__ldg((const S *)((const char *)fq[q] + off))); }
+    __device__ __forceinline__ C full(int q, unsigned off) const { if constexpr (Storage<S>::dev) return val(q, off) + ref(q); else return val(q, off); }
+    static constexpr unsigned EB = sizeof(S);
     __device__ __forceinline__ static C ref(int q) { return Storage<S>::dev ? (C)dev_ref(q) : C(0); }
 
     // Lagrange weights. FP64 takes each node's own: they differ from the first node's by the rounding
@@ -78,24 +81,31 @@ struct Chunk {
 
     __device__ __forceinline__ int base(int t) const { return min(max(t - 3, 0), k.NZ - 7); }
 
+    __device__ __forceinline__ int wrap_x(int v) const {   // v in [-3, NX + W + 2]
+        const int NX = k.NX;
+        if (NX < 8) return wrap_any(v, NX);
+        v = v < 0 ? v + NX : v;
+        v = v >= NX ? v - NX : v;
+        return v >= NX ? v - NX : v;
+    }
+
     // phase A: y filter of 7, 8, 9, 10 on planes p0 .. p0 + np - 1, columns x0 - 3 .. x0 + W + 2
     __device__ __forceinline__ void halo_quads(Quad<C> *qb, int p0, int np, int x0, int y0) const {
         const int WH = cc.W + 6, HW = cc.H*WH, NX = k.NX, NY = k.NY;
-        const size_t N = (size_t)NX*NY*k.NZ;
         for (int i = threadIdx.x; i < np*HW; i += NT) {
-            const int pl = i/HW, r = i - pl*HW, yl = r/WH, xx = r - yl*WH;
+            const int pl = (int)__umulhi((unsigned)i, cc.inv_hw), r = i - pl*HW, yl = (int)__umulhi((unsigned)r, cc.inv_wh), xx = r - yl*WH;
             const int y = y0 + yl;
             if (y >= NY) continue;
-            const S *b = fo + (size_t)(p0 + pl)*NY*NX + wrap_any(x0 + xx - 3, NX);
+            const unsigned b = (unsigned)((p0 + pl)*NY*NX + wrap_x(x0 + xx - 3));
             C s7 = 0, s8 = 0, s9 = 0, s10 = 0;
 #pragma unroll
             for (int j = 0; j < 7; j++) {
-                const S *p = b + (size_t)wrap_near(y - 3 + j, NY)*NX;
+                const unsigned o = (b + (unsigned)(wrap_near(y - 3 + j, NY)*NX))*EB;
                 const C w0 = wy0(j, y), w2 = wy2(j, y);
-                s7 += w0*val(p + 7*N);
-                s8 += w0*val(p + 8*N);
-                s9 += w2*val(p + 9*N);
-                s10 += w2*val(p + 10*N);
+                s7 += w0*val(7, o);
+                s8 += w0*val(8, o);
+                s9 += w2*val(9, o);
+                s10 += w2*val(10, o);
             }
             qb[i] = Quad<C>{s7, s8, s9, s10};
         }
@@ -104,46 +114,42 @@ struct Chunk {
     struct Col {
         int x, y, xl, yl;
         bool on;
-        int xo[7];      // wrapped x of the spanwise stencil
-        int yo[7];      // row offsets (wrapped y times NX) of the streamwise stencil
+        unsigned xo[7];      // byte offsets within a plane: the spanwise stencil's nodes
+        unsigned yo[7];      // and the streamwise stencil's
     };
 
     // phase B: ring values of one column on one plane; ring order 3, 4, 5, 6 | 7, 8, 9, 10 |
     // 11, 12, 13, 14 | 15, 16, 17, 18
     __device__ __forceinline__ void filter(const Col &L, const Quad<C> *qrow, int p, Quad<C> *slot) const {
-        const int NX = k.NX, NY = k.NY;
-        const size_t N = (size_t)NX*NY*k.NZ;
-        const S *pl = fo + (size_t)p*NY*NX;
+        const unsigned pl = (unsigned)(p*k.NY*k.NX)*EB;
         {
-            const S *b = pl + L.x;
             Quad<C> g{0, 0, 0, 0}, h{0, 0, 0, 0};
 #pragma unroll
             for (int j = 0; j < 7; j++) {
-                const S *r = b + L.yo[j];
+                const unsigned o = pl + L.yo[j];
                 const C w0 = wy0(j, L.y), w2 = wy2(j, L.y);
-                g.a += w0*val(r + 3*N);
-                g.b += w2*val(r + 4*N);
-                h.a += w0*val(r + 15*N);
-                h.b += w2*val(r + 16*N);
-                h.c += w0*val(r + 17*N);
-                h.d += w2*val(r + 18*N);
+                g.a += w0*val(3, o);
+                g.b += w2*val(4, o);
+                h.a += w0*val(15, o);
+                h.b += w2*val(16, o);
+                h.c += w0*val(17, o);
+                h.d += w2*val(18, o);
             }
-            g.c = val(b + L.yo[3] + 5*N);
-            g.d = val(b + L.yo[3] + 6*N);
+            g.c = val(5, pl + L.yo[3]);
+            g.d = val(6, pl + L.yo[3]);
             slot[0*P] = g;
             slot[3*P] = h;
         }
         {
-            const S *b = pl + L.yo[3];
             Quad<C> g{0, 0, 0, 0}, h{0, 0, 0, 0};
 #pragma unroll
             for (int a = 0; a < 7; a++) {
-                const S *r = b + L.xo[a];
+                const unsigned o = pl + L.xo[a];
                 const C w0 = wx0(a, L.x), w2 = wx2(a, L.x);
-                h.a += w0*val(r + 11*N);
-                h.b += w2*val(r + 12*N);
-                h.c += w0*val(r + 13*N);
-                h.d += w2*val(r + 14*N);
+                h.a += w0*val(11, o);
+                h.b += w2*val(12, o);
+                h.c += w0*val(13, o);
+                h.d += w2*val(14, o);
                 const Quad<C> v = qrow[a];
                 g.a += w0*v.a;
                 g.b += w2*v.b;
@@ -175,7 +181,6 @@ struct Chunk {
         __shared__ int count;
         __shared__ unsigned short list[2*P*8];
         const int WH = cc.W + 6, NX = k.NX, NY = k.NY, nb = 2*k.NYD6;
-        const size_t N = (size_t)NX*NY*k.NZ;
         if (threadIdx.x == 0) count = 0;
         __syncthreads();
         for (int i = z0*cc.H*8 + threadIdx.x; i < z1*cc.H*8; i += NT) {
@@ -188,7 +193,8 @@ struct Chunk {
             const int e = list[i/WH], xx = i % WH, kd = e & 7, fl = kind_flag(kd), q = kind_src(kd);
             const int z = e/(8*cc.H), y = y0 + (e/8) % cc.H, r = z*k.NYD6 + y + 3;
             const int iy = k.bfl_mode ? r : y + 3;   // reference: Y weights at [j]
-            const S *b = fo + (size_t)q*N + wrap_any(x0 + xx - 3, NX);
+            const unsigned b = (unsigned)wrap_x(x0 + xx - 3);
+            const S *f = fq[q];
             const C rq = ref(q);
             C wy[7], sum = 0;
 #pragma unroll
@@ -197,7 +203,11 @@ struct Chunk {
             for (int c = 0; c < 7; c++) {
                 C in = 0;
 #pragma unroll
-                for (int j = 0; j < 7; j++) in += full(b + ((size_t)c*NY + wrap_near(y - 3 + j, NY))*NX, rq)*wy[j];
+                for (int j = 0; j < 7; j++) {
+                    const C v = to_c(__ldg(f + (b + (unsigned)((c*NY + wrap_near(y - 3 + j, NY))*NX))));
+                    if constexpr (Storage<S>::dev) in += (v + rq)*wy[j];
+                    else in += v*wy[j];
+                }
                 sum += in*bw(kind_zset(fl), c, r);
             }
             bf[(size_t)e*WH + xx] = sum;
@@ -206,13 +216,12 @@ struct Chunk {
 
     __device__ __forceinline__ void bfl_apply(C (&F)[19], const Col &L, int z, const C *bf) const {
         const int NX = k.NX, NY = k.NY, nb = 2*k.NYD6, WH = cc.W + 6;
-        const size_t N = (size_t)NX*NY*k.NZ;
         const int r = z*k.NYD6 + L.y + 3;
         const int ix = k.bfl_mode ? r : L.x + 3;   // reference: X weights at [i]
-        const S *nd = fo + ((size_t)z*NY + L.y)*NX + L.x;
+        const unsigned nd = (unsigned)((z*NY + L.y)*NX + L.x)*EB;
         const C *row = bf + (size_t)(z*cc.H + L.yl)*8*WH + L.xl;
         auto lin = [&](C q, int a, int b) -> C {   // (1/(2Q)) f_a + ((2Q-1)/(2Q)) f_b at the node
-            return (C(1)/(C(2)*q))*full(nd + a*N, ref(a)) + ((C(2)*q - C(1))/(C(2)*q))*full(nd + b*N, ref(b));
+            return (C(1)/(C(2)*q))*full(a, nd) + ((C(2)*q - C(1))/(C(2)*q))*full(b, nd);
         };
         auto xf = [&](int kd, int set) -> C {
             C s = 0;
@@ -247,7 +256,6 @@ struct Chunk {
     __device__ __forceinline__ void target(const Col &L, const Quad<C> *ring, int t, const C *bf, C f6, C f12, C rho_mod,
                                            double &ub, double &mass) const {
         const int NX = k.NX, NY = k.NY;
-        const size_t N = (size_t)NX*NY*k.NZ;
         const int b = base(t);
         C F[19];
         {
@@ -270,29 +278,28 @@ struct Chunk {
 #pragma unroll
             for (int j = 0; j < 16; j++) F[3 + j] = a[j];
         }
-        const size_t node = ((size_t)t*NY + L.y)*NX + L.x;
+        const unsigned node = (unsigned)((t*NY + L.y)*NX + L.x), nd = node*EB;
         {
-            const S *r = fo + (size_t)t*NY*NX + L.yo[3];
+            const unsigned pl = (unsigned)(t*NY*NX)*EB;
             C s1 = 0, s2 = 0;
 #pragma unroll
-            for (int a = 0; a < 7; a++) { s1 += wx0(a, L.x)*val(r + L.xo[a] + N); s2 += wx2(a, L.x)*val(r + L.xo[a] + 2*N); }
+            for (int a = 0; a < 7; a++) { s1 += wx0(a, L.x)*val(1, pl + L.xo[a]); s2 += wx2(a, L.x)*val(2, pl + L.xo[a]); }
             F[1] = s1; F[2] = s2;
-            F[0] = val(fo + node);
+            F[0] = val(0, nd);
         }
         if constexpr (Storage<S>::dev) {
 #pragma unroll
             for (int q = 0; q < 19; q++) F[q] = F[q] + ref(q);
         }
-        const S *nd = fo + node;
-        auto opp = [&](int q) -> C { return full(nd + q*N, ref(q)); };
+        auto opp = [&](int q) -> C { return full(q, nd); };
         if (t == 0) { F[5] = opp(6); F[11] = opp(14); F[12] = opp(13); F[15] = opp(18); F[16] = opp(17); }
         if (t == k.NZ - 1) { F[6] = opp(5); F[13] = opp(12); F[14] = opp(11); F[17] = opp(16); F[18] = opp(15); }
         if (t <= 1) bfl_apply(F, L, t, bf);
         C rho, u1, v1, w1;
-        if constexpr (std::is_same<S, float>::value) collide_pairs<C, LES>(F, rho_mod, f6, f12, (C)k.tau, (C)k.les_C, rho, u1, v1, w1);
+        if constexpr (sizeof(C) == 4) collide_node<C, LES>(F, rho_mod, f6, f12, (C)k.tau, (C)k.les_C, rho, u1, v1, w1);
         else collide<LES>(F, rho_mod, f6, f12, (C)k.tau, (C)k.les_C, rho, u1, v1, w1);
 #pragma unroll
-        for (int q = 0; q < 19; q++) store_f<S>(fn + (size_t)q*N, node, q, F[q]);
+        for (int q = 0; q < 19; q++) store_f<S>((S *)((char *)fnq[q] + nd), 0, q, F[q]);
         if (macros_on) { rho_out[node] = rho; u_out[node] = u1; v_out[node] = v1; w_out[node] = w1; }
         if (L.y == k.yplane) ub += (double)v1*T.dxv[L.x]*T.dzv[t];
         if (mass_on) mass += (double)rho;
@@ -319,8 +326,8 @@ struct Chunk {
             if (L.on) {
 #pragma unroll
                 for (int a = 0; a < 7; a++) {
-                    L.xo[a] = wrap_any(L.x - 3 + a, NX);
-                    L.yo[a] = wrap_near(L.y - 3 + a, NY)*NX;
+                    L.xo[a] = (unsigned)(L.y*NX + wrap_any(L.x - 3 + a, NX))*EB;
+                    L.yo[a] = (unsigned)(wrap_near(L.y - 3 + a, NY)*NX + L.x)*EB;
                 }
             }
             int np = base(ta);   // next plane to filter
@@ -376,8 +383,8 @@ template <class S, bool LES>
 cudaError_t launch_t(const StepLaunch &L) {
     using C = typename Storage<S>::C;
     Chunk<S, LES> K;
-    K.fo = (const S *)L.fo;
-    K.fn = (S *)L.fn;
+    const size_t N = (size_t)L.k.NX*L.k.NY*L.k.NZ;
+    for (int q = 0; q < 19; q++) { K.fq[q] = (const S *)L.fo + q*N; K.fnq[q] = (S *)L.fn + q*N; }
     K.T = *(const Tables<C> *)L.tables;
     K.k = L.k;
     K.cc = *(const ChunkConst *)L.chunk;
@@ -394,15 +401,19 @@ cudaError_t launch_t(const StepLaunch &L) {
 
 template <class F>
 cudaError_t by_kernel(int precision, bool les, F &&f) {
-    switch (precision) {
-    case ISLBM_FP64: return les ? f((double *)nullptr, std::true_type{}) : f((double *)nullptr, std::false_type{});
-    case ISLBM_FP32: return les ? f((float *)nullptr, std::true_type{}) : f((float *)nullptr, std::false_type{});
-    case ISLBM_FP16_DEV: return les ? f((__half *)nullptr, std::true_type{}) : f((__half *)nullptr, std::false_type{});
-    default: return les ? f((__nv_bfloat16 *)nullptr, std::true_type{}) : f((__nv_bfloat16 *)nullptr, std::false_type{});
-    }
+    if (precision == ISLBM_FP64) return les ? f((double *)nullptr, std::true_type{}) : f((double *)nullptr, std::false_type{});
+    return les ? f((float *)nullptr, std::true_type{}) : f((float *)nullptr, std::false_type{});
 }
 
 }  // namespace
+
+bool chunk_supported(const StepConst &k, int precision) {
+    // 16-bit storage keeps the gather kernel's order of summation: each changed rounding of a stored value
+    // is a visible change there
+    if (precision != ISLBM_FP64 && precision != ISLBM_FP32) return false;
+    const double elem = precision == ISLBM_FP64 ? 8 : 4;
+    return (double)k.NX*k.NY*k.NZ*elem < 4294967296.0;
+}
 
 cudaError_t make_chunk_const(const StepConst &k, int precision, bool les, const double *wx0, const double *wx2,
                              const double *wy0, const double *wy2, int num_sms, ChunkConst *out) {
@@ -420,6 +431,8 @@ cudaError_t make_chunk_const(const StepConst &k, int precision, bool les, const 
         if (cost < best*(1.0 - 1e-9)) { best = cost; cc.W = W; cc.H = H; cc.tiles_x = tx; cc.tiles_y = ty; }
         if (W <= 4) break;
     }
+    cc.inv_hw = (unsigned)((0x100000000ULL + cc.H*(cc.W + 6) - 1)/(cc.H*(cc.W + 6)));
+    cc.inv_wh = (unsigned)((0x100000000ULL + cc.W + 5)/(cc.W + 6));
     cc.smem_bytes = precision == ISLBM_FP64 ? smem_for<double>(cc.W, cc.H) : smem_for<float>(cc.W, cc.H);
     int ctas = 0;
     cudaError_t e = by_kernel(precision, les, [&](auto *s, auto l) {

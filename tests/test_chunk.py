@@ -1,6 +1,7 @@
-"""The chunk-marching step kernel (FP64 on every grid, the other formats on grids without a tiled
-layout) where its tiles, chunks and segments have edges: widths below, at and above the 32 lanes of
-a tile, odd counts in every direction, the smallest column, partial tiles, both BFL table modes.
+"""The chunk-marching step kernel (FP64 on every grid, FP32 on grids without a tiled layout; the 16-bit
+formats keep the gather kernel there) where its tiles, chunks and segments have edges: widths below, at
+and above the 32 lanes of a tile, odd counts in every direction, the smallest column, partial tiles, both
+BFL table modes.
 
 FP64 against the oracle: both evaluate the same sums in another order; a step's relative rounding
 difference is a few 1e-16 and grows at most in proportion to the steps here, so 1e-12 holds. The

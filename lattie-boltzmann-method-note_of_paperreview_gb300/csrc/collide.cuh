@@ -13,9 +13,9 @@
 //     force in the odd part;
 //   * Smagorinsky: tau* = tau + 3 C |S| with |S| = (sqrt(nu0^2 + 18 C sqrt(Q)) - nu0)/(6 C), that is
 //     tau* = tau + (sqrt(nu0^2 + 18 C sqrt(Q)) - nu0)/2: two square roots and one reciprocal.
-// FP64 and the 16-bit formats use it. FP32 storage keeps the moment-by-moment forms (collide_pairs,
-// collide_x2), whose rounding biases the flow by up to 2e-5 in the velocity over the runs compared
-// (2.7e-6 with this one): FP32 runs continue what earlier ones gave.
+// FP64 uses it. FP32 arithmetic keeps the moment-by-moment forms (collide_node, collide_pairs,
+// collide_x2): their rounding biases the flow by up to 2e-5 in the velocity over the runs compared
+// (2.7e-6 with this one), and FP32 and 16-bit runs are to continue what earlier ones gave.
 // About 180 operations per node (with the closure 195) against 270 of the moment-by-moment form.
 #pragma once
 
@@ -38,11 +38,8 @@ __device__ __forceinline__ float c_rcp(float v) {
     return r;
 }
 
-// F: streamed populations on entry, post-collision ones on exit. R: the scalar type of T. DEV: F holds
-// the deviations from the reference state r_q = dev_ref(q) (rho = 1, u = (0, u0, 0)); its moments
-// enter as constants (they cancel in everything not named k.. below), so the deviation formats need
-// no 38 additions that restore and remove r_q, and sums of small numbers round less.
-template <bool LES, bool DEV = false, class T, class R>
+// F: streamed populations on entry, post-collision ones on exit. R: the scalar type of T.
+template <bool LES, class T, class R>
 __device__ __forceinline__ void collide(T (&F)[19], R rho_modify, R f6, R f12, R tau, R lesC, T &rho, T &u1, T &v1, T &w1) {
     constexpr double se = 1.19, seps = 1.4, sq = 1.2, spi = 1.4, sm = 1.5;
     F[0] = F[0] + T(rho_modify);
@@ -52,36 +49,17 @@ __device__ __forceinline__ void collide(T (&F)[19], R rho_modify, R f6, R f12, R
     const T A5 = F[11] - F[14], A6 = F[12] - F[13], A7 = F[15] - F[18], A8 = F[16] - F[17];
     const T a = S3 + S4, b = S5 + S6, c = S7 + S8;             // diagonals of the xy, xz, yz planes
     const T d34 = A3 - A4, s34 = A3 + A4, d56 = A5 - A6, s56 = A5 + A6, d78 = A7 - A8, s78 = A7 + A8;
-    const T rs = (F[0] + ((S0 + S1) + S2)) + ((a + b) + c);
-    const T jx = (A0 + d34) + d56, js = (A1 + s34) + d78, jz = (A2 + s56) + s78;
-    T jy;
-    if constexpr (DEV) {
-        rho = rs + T(R(1));
-        jy = js + T(R(0.05));
-    } else {
-        rho = rs;
-        jy = js;
-    }
+    rho = (F[0] + ((S0 + S1) + S2)) + ((a + b) + c);
+    const T jx = (A0 + d34) + d56, jy = (A1 + s34) + d78, jz = (A2 + s56) + s78;
     const T inv = c_rcp(rho);
     u1 = T(jx*inv); v1 = T(jy*inv); w1 = T(jz*inv);
     // non-equilibrium parts
     const T xx = T(jx*u1), yy = T(jy*v1), zz = T(jz*w1);
-    const T bp = T(R(1.0/9.0))*rs - T(R(1.0/6.0))*((xx + yy) + zz);
-    T bx = bp, by = bp, d0 = F[0] - T(R(3))*bp, cc = c, amb = a - b;
-    if constexpr (DEV) {
-        constexpr double u0 = 0.05, uu = u0*u0;
-        // pair sums of r_q: axes x (and z) and y, the three diagonals
-        constexpr double kx = (1.0 - 1.5*uu)/9.0, ky = (1.0 + 3.0*uu)/9.0, ka = (1.0 + 3.0*uu)/9.0, kb = (1.0 - 1.5*uu)/9.0, kc = ka;
-        bx = bp + T(R(1.0/9.0 - kx));
-        by = bp + T(R(1.0/9.0 - ky));
-        d0 = d0 - T(R(0.5*uu));                      // 1/3 - r_0
-        if constexpr (kc != ky) cc = c + T(R(kc - ky));
-        if constexpr (ka - kb - ky + kx != 0.0) amb = amb + T(R(ka - kb - ky + kx));
-    }
-    const T X = T(R(0.5))*xx + bx, Y = T(R(0.5))*yy + by, Z = T(R(0.5))*zz + bx;
-    const T x = S0 - X, y = S1 - Y, z = S2 - Z;
-    const T cn = cc - (T(R(0.5))*zz + Y);
-    const T ab = amb - (Y - Z);
+    const T bp = T(R(1.0/9.0))*rho - T(R(1.0/6.0))*((xx + yy) + zz);
+    const T X = T(R(0.5))*xx + bp, Y = T(R(0.5))*yy + bp, Z = T(R(0.5))*zz + bp;
+    const T x = S0 - X, y = S1 - Y, z = S2 - Z, d0 = F[0] - T(R(3))*bp;
+    const T cn = c - (T(R(0.5))*zz + Y);
+    const T ab = (a - b) - (Y - Z);
     const T mxy = (S3 - S4) - jx*v1, mxz = (S5 - S6) - jx*w1, myz = (S7 - S8) - jy*w1;
     const T AX = (x + y) + z;
     const T d1 = x - cn, sd = y - z, pww = sd + ab;
@@ -115,7 +93,7 @@ __device__ __forceinline__ void collide(T (&F)[19], R rho_modify, R f6, R f12, R
     const T ex = T(R(2))*t + e1, eyz = e1 - t, ey = eyz + q, ez = eyz - q;
     const T eg = e2 + g, exy = eg + k, exz = eg - k, ed = e2 - T(R(2))*g;
     // odd part: q from the axis differences, the antisymmetric third-order moments, the force
-    const T dx = A0 - T(R(1.0/3.0))*jx, dy = A1 - T(R(1.0/3.0))*js, dz = A2 - T(R(1.0/3.0))*jz;
+    const T dx = A0 - T(R(1.0/3.0))*jx, dy = A1 - T(R(1.0/3.0))*jy, dz = A2 - T(R(1.0/3.0))*jz;
     const T r4 = T(T(R(-0.125*sq))*dx), r6 = T(T(R(-0.125*sq))*dy), r8 = T(T(R(-0.125*sq))*dz);
     const T m16 = d34 - d56, m17 = d78 - s34, m18 = s56 - s78;
     const T al = T(R(0.125*sm))*m16 + r4, al2 = r4 - T(R(0.125*sm))*m16;

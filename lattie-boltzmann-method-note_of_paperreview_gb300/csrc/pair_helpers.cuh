@@ -71,13 +71,6 @@ template <class S> __device__ __forceinline__ void st2(S *p, V2 v, int q) {
     }
 }
 
-// store a node pair as it is held
-template <class S> __device__ __forceinline__ void st2s(S *p, V2 v) {
-    if constexpr (std::is_same<S, float>::value) *(float2 *)p = v.v;
-    else if constexpr (std::is_same<S, __half>::value) *(__half2 *)p = __float22half2_rn(v.v);
-    else *(__nv_bfloat162 *)p = __float22bfloat162_rn(v.v);
-}
-
 // Tensor copy of one box (x, y, z, q) of a population buffer: the box lands in shared memory as
 // [q][rows][NX], the layout of the front and stage buffers.
 __device__ __forceinline__ void tma_load4(void *dst, const CUtensorMap *map, int x, int y, int z, int q, uint64_t *bar) {

@@ -101,7 +101,10 @@ __device__ __forceinline__ void collide_x2(V2 (&F)[19], float rho_modify, float 
 #pragma unroll
         for (int l = 0; l < 2; l++) {
             const float q = l == 0 ? Qn.v.x : Qn.v.y;
-            const float Sm = __fdividef(sqrt_nn(nu0*nu0 + 18.f*lesC*sqrt_nn(q)) - nu0, 6.f*lesC);
+            // the fused multiply-add is spelled out: which of the two products the compiler fuses would
+            // depend on the kernel around this, and with it the last bit of every LES run
+            const float disc = __fmaf_rn(__fmul_rn(18.f, lesC), sqrt_nn(q), __fmul_rn(nu0, nu0));
+            const float Sm = __fdividef(sqrt_nn(disc) - nu0, 6.f*lesC);
             sn[l] = __fdividef(1.f, tau + 3.f*lesC*Sm);
         }
         s_nu = V2(sn[0], sn[1]);

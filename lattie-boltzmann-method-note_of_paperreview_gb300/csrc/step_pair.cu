@@ -197,8 +197,7 @@ struct PairKernel {
             }
         }
         V2 rho, u1, v1, w1;
-        if constexpr (Storage<S>::dev) collide<LES>(F, sc.rho_mod, sc.f6, sc.f12, sc.tau, sc.lesC, rho, u1, v1, w1);
-        else collide_x2<LES>(F, sc.rho_mod, sc.f6, sc.f12, sc.tau, sc.lesC, rho, u1, v1, w1);
+        collide_x2<LES>(F, sc.rho_mod, sc.f6, sc.f12, sc.tau, sc.lesC, rho, u1, v1, w1);
 #pragma unroll
         for (int q = 0; q < 19; q++) st2<S>(fnq[q] + node, F[q], q);
         if (macros_on) {

@@ -1,6 +1,7 @@
 // Host side of the role-specialised paired kernel (step_roles.cuh): dispatch by storage format, width
 // and closure, column split, tensor maps.
 #include <algorithm>
+#include <cstdlib>
 #include <cstring>
 
 #include "step_roles.hpp"
@@ -58,6 +59,10 @@ cudaError_t make_roles_const(const StepConst &k, int precision, bool les, const 
     tc.TY = 512/k.NX;
     const int tiles = (k.NY + tc.TY - 1)/tc.TY;
     split_columns(tiles, num_sms, k.NZ, tc);
+    if (const char *e = std::getenv("ISLBM_TILED_ZSEGS")) {   // tuning override: equal segments
+        const int z = std::atoi(e);
+        if (z >= 1 && z <= k.NZ/8) { tc.zmain = 0; tc.zlen = 0; tc.zsegs = z; }
+    }
     const long long items = (long long)tiles*(tc.zmain + tc.zsegs);
     tc.grid = tc.zmain ? num_sms : (int)std::min<long long>(items, num_sms);
     tc.seats = tc.grid == num_sms;

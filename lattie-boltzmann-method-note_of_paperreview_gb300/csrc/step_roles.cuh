@@ -46,7 +46,8 @@ constexpr int THREADS = 640;          // five warpgroups: collide, collide, row 
 constexpr int ACTIVE_THREADS = 32*(TARGET_WARP + 1);
 // registers per thread of the warpgroups after the split: two collide groups, row filter, quad filter,
 // producers, together at most the 5*96 that the CTA is launched with
-template <class S> struct Regs { static constexpr int collide = 144, rows = 80, quads = 80, copies = 32; };   // 16-bit formats
+// (16-bit formats, LES, 128x256x192: 152/72/72 205.9 us per step, 144/80/80 217.6, 160/64/64 207.4)
+template <class S> struct Regs { static constexpr int collide = 152, rows = 72, quads = 72, copies = 32; };
 template <> struct Regs<float> { static constexpr int collide = 152, rows = 80, quads = 64, copies = 32; };
 constexpr int SLOTS = 8;              // ring planes
 
@@ -475,21 +476,12 @@ struct RoleKernel {
         else __syncwarp(PR == 32 ? 0xffffffffu : (0xffffu << (threadIdx.x & 16)));
     }
 
-    // a full value as the state holds it (the deviation formats: f - ref)
-    __device__ __forceinline__ static V2 stored(V2 v, int q) {
-        if constexpr (Storage<S>::dev) return v - V2((float)dev_ref(q));
-        else return v;
-    }
-    // half-way bounce-back: population q of a node from its opposite qs (deviations differ by the
-    // difference of their reference values)
-    __device__ __forceinline__ static V2 opposite(const S *node, size_t N, int qs, int q) { return stored(ld2g<S>(node + qs*N, qs), q); }
-
     // One flag type of the BFL rows (C/evolution.h:505-572) of a whole row y at plane z <= 1, called
     // by the row's threads together. dst / src: populations set and their opposites, the first without
     // and the other two with an x filter (n = 1 or 3); wall distance below one half: 7 x 7 (y, xi) sums
     // of the opposite populations per node, exchanged through `sums` for the x filter (a sum of
     // 7 x 7 x 7 terms per thread otherwise).
-    // Returns whether the row is set, with the populations as the state holds them in out.
+    // Returns whether the row is set, with the populations (full values) in out.
     template <int N3>
     __device__ __forceinline__ bool bfl_type(V2 *out, int fl, const int (&dst)[N3], const int (&src)[N3], const int (&xset)[N3],
                                              int yset, int zset, int x0, int y, int z, int row, float *sums) const {
@@ -501,7 +493,7 @@ struct RoleKernel {
             const S *nd = fo + ((size_t)z*NY + y)*NX + x0;
             const float c0 = 1.f/(2.f*q), c1 = (2.f*q - 1.f)/(2.f*q);
 #pragma unroll
-            for (int m = 0; m < N3; m++) out[m] = stored(V2(c0)*ld2g<S>(nd + src[m]*N, src[m]) + V2(c1)*ld2g<S>(nd + dst[m]*N, dst[m]), dst[m]);
+            for (int m = 0; m < N3; m++) out[m] = V2(c0)*ld2g<S>(nd + src[m]*N, src[m]) + V2(c1)*ld2g<S>(nd + dst[m]*N, dst[m]);
         }
         if (q < 0.5f) {
             const int iy = k.bfl_mode ? r : y + 3;   // reference: X weights at [i], Y weights at [j]
@@ -526,7 +518,7 @@ struct RoleKernel {
 #pragma unroll
                 for (int m = 0; m < N3; m++) g[m] = wz*in[m] + g[m];
             }
-            out[0] = stored(g[0], dst[0]);
+            out[0] = g[0];
             if constexpr (N3 == 3) {
                 float *s = sums + row*NX;   // [2][512]: two populations
                 row_sync(row);              // the row's previous sums have been read
@@ -543,7 +535,7 @@ struct RoleKernel {
 #pragma unroll
                         for (int a = 0; a < 7; a++) o[l] += bw(xset[m], a, ix)*s[(m - 1)*512 + ((x0 + l - 3 + a) & (NX - 1))];
                     }
-                    out[m] = stored(V2(o[0], o[1]), dst[m]);
+                    out[m] = V2(o[0], o[1]);
                 }
             }
         }
@@ -563,11 +555,11 @@ struct RoleKernel {
         const size_t N = (size_t)NX*k.NY*k.NZ;
         if (z0 == 0) {
             const S *b = fo + ((size_t)y*NX + x0);
-            w.bounce[0] = opposite(b, N, 6, 5);
-            w.bounce[1] = opposite(b, N, 14, 11);
-            w.bounce[2] = opposite(b, N, 13, 12);
-            w.bounce[3] = opposite(b, N, 18, 15);
-            w.bounce[4] = opposite(b, N, 17, 16);
+            w.bounce[0] = ld2g<S>(b + 6*N, 6);
+            w.bounce[1] = ld2g<S>(b + 14*N, 14);
+            w.bounce[2] = ld2g<S>(b + 13*N, 13);
+            w.bounce[3] = ld2g<S>(b + 18*N, 18);
+            w.bounce[4] = ld2g<S>(b + 17*N, 17);
         }
 #pragma unroll 1
         for (int z = z0; z < z1; z++) {
@@ -581,7 +573,7 @@ struct RoleKernel {
     }
 
     // Walls, BFL rows, collision and stores of the node pair (x0, x0 + 1) at row y, plane z, whose
-    // streamed populations are in F as the state holds them (deviations for the deviation formats)
+    // streamed populations are in F (deviations for the deviation formats)
     // (WALL: z <= 1, the planes that the lower wall sets)
     template <bool WALL>
     __device__ __forceinline__ void finish(V2 (&F)[19], int x0, int y, int z, const Scal &sc, float &ub, V2 &mass, const Wall *wall) const {
@@ -591,6 +583,10 @@ struct RoleKernel {
         // instead of a 64-bit address each (FP16 193 -> 182 us per step on 256x128x192)
         const unsigned node = (unsigned)((z*NY + y)*NX + x0), off = node*(unsigned)sizeof(S), moff = node*4u;
         const S *b = (const S *)((const char *)fo + off);
+        if constexpr (Storage<S>::dev) {
+#pragma unroll
+            for (int q = 0; q < 19; q++) F[q] = F[q] + V2((float)dev_ref(q));
+        }
         if constexpr (WALL) {
             if (z == 0) { F[5] = wall->bounce[0]; F[11] = wall->bounce[1]; F[12] = wall->bounce[2]; F[15] = wall->bounce[3]; F[16] = wall->bounce[4]; }
             const V2 *v = wall->v[z];
@@ -601,14 +597,13 @@ struct RoleKernel {
             if (m & 8u) F[16] = v[7];
         }
         if (z == k.NZ - 1) {
-            F[6] = opposite(b, N, 5, 6); F[13] = opposite(b, N, 12, 13); F[14] = opposite(b, N, 11, 14);
-            F[17] = opposite(b, N, 16, 17); F[18] = opposite(b, N, 15, 18);
+            F[6] = ld2g<S>(b + 5*N, 5); F[13] = ld2g<S>(b + 12*N, 12); F[14] = ld2g<S>(b + 11*N, 11);
+            F[17] = ld2g<S>(b + 16*N, 16); F[18] = ld2g<S>(b + 15*N, 15);
         }
         V2 rho, u1, v1, w1;
-        if constexpr (Storage<S>::dev) collide<LES, true>(F, sc.rho_mod, sc.f6, sc.f12, sc.tau, sc.lesC, rho, u1, v1, w1);
-        else collide_x2<LES>(F, sc.rho_mod, sc.f6, sc.f12, sc.tau, sc.lesC, rho, u1, v1, w1);
+        collide_x2<LES>(F, sc.rho_mod, sc.f6, sc.f12, sc.tau, sc.lesC, rho, u1, v1, w1);
 #pragma unroll
-        for (int q = 0; q < 19; q++) st2s<S>((S *)((char *)fnq[q] + off), F[q]);
+        for (int q = 0; q < 19; q++) st2<S>((S *)((char *)fnq[q] + off), F[q], q);
         if (macros_on) {
             *(float2 *)((char *)rho_out + moff) = rho.v; *(float2 *)((char *)u_out + moff) = u1.v;
             *(float2 *)((char *)v_out + moff) = v1.v; *(float2 *)((char *)w_out + moff) = w1.v;

@@ -201,7 +201,8 @@ int islbm_stats_mean(islbm_handle *h, int quantity, double *out, int layout) {
     const double inv = 1.0/(double)h->stats_samples;
     std::vector<double> mean(layout == ISLBM_LAYOUT_REFERENCE ? h->N : 0);
     double *dst = mean.empty() ? out : mean.data();
-    e = handle_xfer(h);
+    double *direct = mean.empty() ? pinned_device_alias(out, h->N) : nullptr;
+    e = direct ? cudaSuccess : handle_xfer(h);
     if (e == cudaErrorMemoryAllocation) {   // no device memory for the buffer: scaled on the host
         (void)cudaGetLastError();
         e = cudaMemcpyAsync(dst, h->stats + (size_t)quantity*h->N, h->N*sizeof(double), cudaMemcpyDeviceToHost, h->stream);
@@ -210,9 +211,9 @@ int islbm_stats_mean(islbm_handle *h, int quantity, double *out, int layout) {
             for (size_t i = 0; i < h->N; i++) dst[i] *= inv;
     } else if (e == cudaSuccess) {
         const unsigned grid = (unsigned)std::min<size_t>(4096, (h->N + 255)/256);
-        mean_kernel<<<grid, 256, 0, h->stream>>>(h->stats + (size_t)quantity*h->N, h->xfer, h->N, inv);
+        mean_kernel<<<grid, 256, 0, h->stream>>>(h->stats + (size_t)quantity*h->N, direct ? direct : h->xfer, h->N, inv);
         e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaMemcpyAsync(dst, h->xfer, h->N*sizeof(double), cudaMemcpyDeviceToHost, h->stream);
+        if (e == cudaSuccess && !direct) e = cudaMemcpyAsync(dst, h->xfer, h->N*sizeof(double), cudaMemcpyDeviceToHost, h->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     }
     if (e != cudaSuccess) return report_cuda(e, "statistics read");

@@ -62,7 +62,7 @@ typedef enum islbm_layout {
 } islbm_layout;
 
 typedef enum islbm_kernel {
-    ISLBM_KERNEL_AUTO = 0,       /* tiled kernel when the grid allows it, else gather kernel */
+    ISLBM_KERNEL_AUTO = 0,       /* the fastest kernel for the grid and storage format */
     ISLBM_KERNEL_GATHER = 1,     /* one thread per node, stencils read through L1/L2 */
     ISLBM_KERNEL_TILED = 2,      /* z-marching x-y tiles staged in shared memory (two nodes per
                                     thread where the width allows it, else one) */

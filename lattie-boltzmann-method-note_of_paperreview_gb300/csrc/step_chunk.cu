@@ -65,12 +65,10 @@ struct Chunk {
     C ux0[7], ux2[7], uy0[7], uy2[7];   // FP32: uniform spacing, the weights of the first node
     int macros_on, mass_on;
 
-    // stored value (a deviation for FP16 / BF16) of population q at a byte offset (chunk_supported: 32 bits).
+    // value of population q at a byte offset (chunk_supported: 32 bits).
     // 64-bit addresses, one per load, were 40% of the kernel's instructions (FP32 187x91x131 224 us per step).
     __device__ __forceinline__ C val(int q, unsigned off) const { return to_c(__ldg((const S *)((const char *)fq[q] + off))); }
-    __device__ __forceinline__ C full(int q, unsigned off) const { if constexpr (Storage<S>::dev) return val(q, off) + ref(q); else return val(q, off); }
     static constexpr unsigned EB = sizeof(S);
-    __device__ __forceinline__ static C ref(int q) { return Storage<S>::dev ? (C)dev_ref(q) : C(0); }
 
     // Lagrange weights. FP64 takes each node's own: they differ from the first node's by the rounding
     // of the node positions (about 1e-14), which the 1e-12 parity over a thousand steps would see
@@ -195,7 +193,6 @@ struct Chunk {
             const int iy = k.bfl_mode ? r : y + 3;   // reference: Y weights at [j]
             const unsigned b = (unsigned)wrap_x(x0 + xx - 3);
             const S *f = fq[q];
-            const C rq = ref(q);
             C wy[7], sum = 0;
 #pragma unroll
             for (int j = 0; j < 7; j++) wy[j] = bw(kind_yset(fl), j, iy);
@@ -204,9 +201,7 @@ struct Chunk {
                 C in = 0;
 #pragma unroll
                 for (int j = 0; j < 7; j++) {
-                    const C v = to_c(__ldg(f + (b + (unsigned)((c*NY + wrap_near(y - 3 + j, NY))*NX))));
-                    if constexpr (Storage<S>::dev) in += (v + rq)*wy[j];
-                    else in += v*wy[j];
+                    in += to_c(__ldg(f + (b + (unsigned)((c*NY + wrap_near(y - 3 + j, NY))*NX))))*wy[j];
                 }
                 sum += in*bw(kind_zset(fl), c, r);
             }
@@ -221,7 +216,7 @@ struct Chunk {
         const unsigned nd = (unsigned)((z*NY + L.y)*NX + L.x)*EB;
         const C *row = bf + (size_t)(z*cc.H + L.yl)*8*WH + L.xl;
         auto lin = [&](C q, int a, int b) -> C {   // (1/(2Q)) f_a + ((2Q-1)/(2Q)) f_b at the node
-            return (C(1)/(C(2)*q))*full(a, nd) + ((C(2)*q - C(1))/(C(2)*q))*full(b, nd);
+            return (C(1)/(C(2)*q))*val(a, nd) + ((C(2)*q - C(1))/(C(2)*q))*val(b, nd);
         };
         auto xf = [&](int kd, int set) -> C {
             C s = 0;
@@ -287,11 +282,7 @@ struct Chunk {
             F[1] = s1; F[2] = s2;
             F[0] = val(0, nd);
         }
-        if constexpr (Storage<S>::dev) {
-#pragma unroll
-            for (int q = 0; q < 19; q++) F[q] = F[q] + ref(q);
-        }
-        auto opp = [&](int q) -> C { return full(q, nd); };
+        auto opp = [&](int q) -> C { return val(q, nd); };
         if (t == 0) { F[5] = opp(6); F[11] = opp(14); F[12] = opp(13); F[15] = opp(18); F[16] = opp(17); }
         if (t == k.NZ - 1) { F[6] = opp(5); F[13] = opp(12); F[14] = opp(11); F[17] = opp(16); F[18] = opp(15); }
         if (t <= 1) bfl_apply(F, L, t, bf);

@@ -47,15 +47,15 @@ template <> __device__ __forceinline__ V2 ld2v<__half>(const __half *p) { return
 template <> __device__ __forceinline__ V2 ld2v<__nv_bfloat16>(const __nv_bfloat16 *p) {
     return V2(__bfloat1622float2(*(const __nv_bfloat162 *)p));
 }
-// full values of a node pair from global memory (read-only path)
+// full values of a node pair from global memory (plain loads: see grid_dependency_wait)
 template <class S> __device__ __forceinline__ V2 ld2g(const S *p, int q) {
     V2 v;
-    if constexpr (std::is_same<S, float>::value) v = V2(__ldg((const float2 *)p));
+    if constexpr (std::is_same<S, float>::value) v = V2(*(const float2 *)p);
     else if constexpr (std::is_same<S, __half>::value) {
-        const unsigned r = __ldg((const unsigned *)p);
+        const unsigned r = *(const unsigned *)p;
         v = V2(__half22float2(*(const __half2 *)&r));
     } else {
-        const unsigned r = __ldg((const unsigned *)p);
+        const unsigned r = *(const unsigned *)p;
         v = V2(__bfloat1622float2(*(const __nv_bfloat162 *)&r));
     }
     if constexpr (Storage<S>::dev) v = v + V2((float)dev_ref(q));

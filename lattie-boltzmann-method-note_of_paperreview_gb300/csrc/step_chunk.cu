@@ -65,9 +65,9 @@ struct Chunk {
     C ux0[7], ux2[7], uy0[7], uy2[7];   // FP32: uniform spacing, the weights of the first node
     int macros_on, mass_on;
 
-    // value of population q at a byte offset (chunk_supported: 32 bits).
+    // value of population q at a byte offset (chunk_supported: 32 bits), by a plain load (grid_dependency_wait).
     // 64-bit addresses, one per load, were 40% of the kernel's instructions (FP32 187x91x131 224 us per step).
-    __device__ __forceinline__ C val(int q, unsigned off) const { return to_c(__ldg((const S *)((const char *)fq[q] + off))); }
+    __device__ __forceinline__ C val(int q, unsigned off) const { return to_c(*(const S *)((const char *)fq[q] + off)); }
     static constexpr unsigned EB = sizeof(S);
 
     // Lagrange weights. FP64 takes each node's own: they differ from the first node's by the rounding
@@ -201,7 +201,7 @@ struct Chunk {
                 C in = 0;
 #pragma unroll
                 for (int j = 0; j < 7; j++) {
-                    in += to_c(__ldg(f + (b + (unsigned)((c*NY + wrap_near(y - 3 + j, NY))*NX))))*wy[j];
+                    in += to_c(f[b + (unsigned)((c*NY + wrap_near(y - 3 + j, NY))*NX)])*wy[j];
                 }
                 sum += in*bw(kind_zset(fl), c, r);
             }
@@ -353,8 +353,9 @@ template <class S> constexpr int min_ctas() { return sizeof(typename Storage<S>:
 template <class S, bool LES>
 __global__ void __launch_bounds__(NT, min_ctas<S>()) step_chunk_kernel(const __grid_constant__ Chunk<S, LES> K) {
     extern __shared__ __align__(128) unsigned char smem[];
-    grid_dependency_trigger();
+    // the trigger comes after the wait: at most two steps are resident at a time
     grid_dependency_wait();
+    grid_dependency_trigger();
     K.run(smem);
 }
 

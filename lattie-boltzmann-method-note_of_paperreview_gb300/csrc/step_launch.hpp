@@ -27,8 +27,13 @@ struct StepLaunch {
 
 // Programmatic dependent launch of consecutive step kernels: the next step's blocks may start, set up
 // their barriers and tensor memory and then wait for the previous step's end and its memory
-// (grid_dependency_wait) while that one's last blocks still run. A kernel launched this way reads and
-// writes nothing in global memory before the wait.
+// (grid_dependency_wait) while that one's last blocks still run. A kernel launched this way touches no
+// global memory before the wait but the seat words (claim_seat in step_roles.cuh: every block of the
+// previous step has claimed its seat before it triggers). Populations are read with plain loads
+// through pointers without __restrict__: the read-only path (__ldg, ld.global.nc) is for memory that
+// nothing writes while the kernel is resident, and the previous step writes them until the wait
+// ends. A read-only line cached by the step before that could be stale, and such a load may be
+// moved above the wait. The tables, written at set-up only, may take that path.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dependency_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <class... P, class... A>

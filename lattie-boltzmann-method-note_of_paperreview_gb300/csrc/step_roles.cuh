@@ -129,8 +129,8 @@ struct RoleKernel {
     static constexpr int NX = NXC, PR = LY::PR, TY = LY::TY;
     static_assert(2*Regs<S>::collide + Regs<S>::rows + Regs<S>::quads + Regs<S>::copies <= 480, "register split");
     struct Scal { float f6, f12, rho_mod, tau, lesC; };
-    const S *__restrict__ fo;
-    S *__restrict__ fn;
+    const S *fo;
+    S *fn;
     S *fnq[19];                // fn + q*N
     Tables<float> T;
     StepConst k;

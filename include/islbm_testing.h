@@ -1,4 +1,4 @@
-/* islbm_testing.h - hooks for testing the failure path of the step kernels.
+/* islbm_testing.h - hooks for testing the step kernels: their failure path and their choice.
  *
  * No reference counterpart. The tiled step kernel waits for its shared-memory copies with
  * bounded waits (about a second); when one runs out, the kernel records the fault in the
@@ -19,6 +19,10 @@ extern "C" {
 /* From the next islbm_step on, the tiled kernel skips the copies of wall-normal plane `plane`
  * (0 <= plane < NZ); -1 turns the drill off. The solve's state is undefined afterwards. */
 ISLBM_API int islbm_fault_drill(islbm_handle *h, int plane);
+
+/* The kernel that steps this solve. */
+enum { ISLBM_STEP_GATHER = 0, ISLBM_STEP_CHUNK = 1, ISLBM_STEP_TILED = 2, ISLBM_STEP_PAIRED = 3, ISLBM_STEP_ROLES = 4 };
+ISLBM_API int islbm_step_kernel(const islbm_handle *h, int *kernel);
 
 #ifdef __cplusplus
 }

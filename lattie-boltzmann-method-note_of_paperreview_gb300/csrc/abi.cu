@@ -510,7 +510,18 @@ int init_impl(const islbm_params *pp, islbm_handle *h) {
         }
         if (p.kernel != ISLBM_KERNEL_AUTO && !h->use_tiled) { g_last = "tiled kernel does not support this grid"; return ISLBM_ERR_NOT_SUPPORTED; }
     }
-    if (p.kernel == ISLBM_KERNEL_AUTO && !h->use_tiled && chunk_supported(k, p.precision)) {
+    // FP32: the chunk kernel gives the gather kernel's bits where a weight has the same FP32 value at every
+    // node (all of 40 grids tried; the FP64 ones differ by the rounding of the node positions)
+    auto one_value = [](const std::vector<double> &w, int stride, int n) {
+        for (int a = 0; a < 7; a++)
+            for (int i = 1; i < n; i++)
+                if ((float)w[(size_t)a*stride + 3 + i] != (float)w[(size_t)a*stride + 3]) return false;
+        return true;
+    };
+    const Geometry &g = h->g;
+    if (p.kernel == ISLBM_KERNEL_AUTO && !h->use_tiled && chunk_supported(k, p.precision) &&
+        (p.precision == ISLBM_FP64 || (one_value(g.XP0, g.NX6, p.NX) && one_value(g.XP2, g.NX6, p.NX) &&
+                                       one_value(g.YP0, g.NYD6, p.NY) && one_value(g.YP2, g.NYD6, p.NY)))) {
         CK(make_chunk_const(k, p.precision, p.les_cs > 0.0, wx0, wx2, wy0, wy2, sms, &h->chunk));
         h->chunked = true;
     }
@@ -733,6 +744,13 @@ int islbm_fault_drill(islbm_handle *h, int plane) {
     if (check_handle(h) || plane < -1 || plane >= h->p.NZ) return ISLBM_ERR_INVALID_ARGUMENT;
     if (!h->use_tiled) { g_last = "the failure drill needs the tiled kernel"; return ISLBM_ERR_NOT_SUPPORTED; }
     h->k.drill_plane = plane;
+    return ISLBM_OK;
+}
+
+int islbm_step_kernel(const islbm_handle *h, int *kernel) {
+    if (check_handle(h) || !kernel) return ISLBM_ERR_INVALID_ARGUMENT;
+    *kernel = h->roles ? ISLBM_STEP_ROLES : h->paired ? ISLBM_STEP_PAIRED : h->use_tiled ? ISLBM_STEP_TILED
+            : h->chunked ? ISLBM_STEP_CHUNK : ISLBM_STEP_GATHER;
     return ISLBM_OK;
 }
 

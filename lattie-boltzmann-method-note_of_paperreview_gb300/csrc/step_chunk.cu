@@ -6,22 +6,25 @@
 // 7 x 7 x 7 stencil by itself: about 2,500 multiply-adds and adds per node. Here the streamwise and
 // spanwise filters are applied once per plane and node and the xi combination once per target,
 // 252 multiply-adds per node, as the tiled kernels do:
-//   * a CTA of 128 threads owns a tile of W x H <= 32 columns (one lane each) and marches upward
-//     through a wall-normal segment in chunks of CHUNK planes;
-//   * phase A filters 7, 8, 9, 10 in y on the chunk's new planes, for the tile's columns and
-//     three halo columns on each side, into shared memory; phase B filters them in x, the other
-//     populations in y or x straight from global memory (L1 / L2), and stores the 16 values of
-//     every column in a ring of CHUNK + 6 planes in shared memory; phase C combines seven planes
-//     per target along xi, collides and stores. The four warps take different planes (A, B)
-//     and targets (C) of a chunk, so a chunk costs two CTA barriers and no other synchronisation;
-//   * bounce-back (BFL) rows: the 7 x 7 (y, xi) sums of the flagged rows are spread over the whole
-//     CTA before phase C, with the halo columns, so that only a 7-tap x filter is left per node.
+//   * a CTA of four groups of threads owns a tile of W x H columns (one lane each of a group: at most 32 in
+//     FP64, 64 in FP32) and marches upward through a wall-normal segment in chunks of CHUNK planes;
+//   * phase A filters 7, 8, 9, 10 along one axis on the chunk's new planes into shared memory: FP64 in y, for the
+//     tile's columns and three halo columns on each side; FP32 in x, for its rows and three halo rows on each
+//     side; phase B filters them along the other axis, the other populations in y or x straight from
+//     global memory (L1 / L2), and stores the 16 values of every column in a ring of CHUNK + 6 planes in
+//     shared memory; phase C combines seven planes per target along xi, collides and stores. The four groups
+//     take different planes (A, B) and targets (C) of a chunk, so a chunk costs two CTA barriers and no
+//     other synchronisation;
+//   * FP32 gives the gather kernel's bits: the same terms in the same order (see GATHER). Populations 3 and 4, whose xi
+//     sums lie inside the y sum, cannot share a filtered plane; four targets share the loads of their windows;
+//   * bounce-back (BFL) rows: the sums of the flagged rows are spread over the whole CTA before phase C.
 //     The gather kernel's per-thread 343-point sums were the critical path on small grids.
 //
-// Bound: in FP64 the FP64 pipe (GB300 issues 2 FP64 lanes per clock and SM: about 560 operations per
-// node take 5.8 ms on 256x128x192); in FP32 the load/store and issue rate. Measured against the
-// gather kernel, per step: FP64 256x128x192 (LES) 28.2 -> 6.97 ms, FP64 64x32x48 506 -> 135 us, FP32
-// 187x91x131 (LES) 2,956 -> 232 us (9.6 GLUPS).
+// Bound: in FP64 the FP64 pipe (GB300 issues 2 FP64 lanes per clock and SM: about 430 operations per
+// node take 4.3 ms on 256x128x192); in FP32 the latency of its loads at 16 warps per SM. Measured against the
+// gather kernel, per step: FP64 256x128x192 (LES) 28.2 -> 5.50 ms, FP64 64x32x48 506 -> 112 us, FP32
+// 187x91x131 (LES) 2,956 -> 272 us (8.2 GLUPS; 182 us with y and xi sums shared by all populations, which
+// changed the last place of the results).
 #include <algorithm>
 #include <type_traits>
 #include <cstring>
@@ -35,13 +38,32 @@ namespace islbm {
 
 namespace {
 
-constexpr int NT = 128, P = 32, GROUPS = NT/P;
+// columns of a tile, one lane each, and the groups of that many lanes that share a CTA's planes and targets
+constexpr int GROUPS = 4;
+template <class C> __host__ __device__ constexpr int lanes() { return sizeof(C) == 4 ? 64 : 32; }
 constexpr int CHUNK = 8, RING = CHUNK + 6;
+// planes filtered between two barriers: a segment's first chunk takes RING, the others CHUNK. FP32 takes that
+// one in two parts, which leaves more of an SM's memory to the L1 cache
+template <class C> __host__ __device__ constexpr int batch() { return sizeof(C) == 4 ? CHUNK : RING; }
+
+// A sum of products, term j = 0, 1, ... (compile-time in unrolled loops). FP32: the roundings that the gather
+// kernel's unrolled sums are compiled to, w0 v0 + round(w1 v1), then one fused term after the other.
+template <class C> struct Sum {
+    C s = 0, w0, v0;
+    __device__ __forceinline__ void add(int j, C w, C v) {
+        if constexpr (sizeof(C) == 8) s += w*v;
+        else if (j == 0) { w0 = w; v0 = v; }
+        else if (j == 1) s = __fmaf_rn(w0, v0, __fmul_rn(w, v));
+        else s = __fmaf_rn(w, v, s);
+    }
+};
 
 // four values of one node (FP32: one 16-byte access, FP64: two)
 template <class C> struct alignas(16) Quad { C a, b, c, d; };
 
-template <class C> __host__ __device__ constexpr size_t ring_bytes() { return (size_t)RING*4*P*sizeof(Quad<C>); }
+template <class C> __host__ __device__ constexpr size_t ring_bytes() { return (size_t)RING*4*lanes<C>()*sizeof(Quad<C>); }
+// FP32: the streamed populations 3 and 4 of a chunk's targets
+template <class C> __host__ __device__ constexpr size_t f34_bytes() { return sizeof(C) == 4 ? (size_t)CHUNK*2*lanes<C>()*sizeof(C) : 0; }
 
 __device__ __forceinline__ int wrap_near(int v, int n) {   // v in [-n, 2n)
     return v < 0 ? v + n : (v >= n ? v - n : v);
@@ -54,6 +76,7 @@ __device__ __forceinline__ int wrap_any(int v, int n) {
 template <class S, bool LES>
 struct Chunk {
     using C = typename Storage<S>::C;
+    static constexpr int P = lanes<C>(), NT = GROUPS*P;
     const S *fq[19];           // old populations, one array each: uniform bases for 32-bit byte offsets
     S *fnq[19];
     Tables<C> T;
@@ -62,8 +85,14 @@ struct Chunk {
     Ctrl *ctrl;
     unsigned long long n;
     C *rho_out, *u_out, *v_out, *w_out;
-    C ux0[7], ux2[7], uy0[7], uy2[7];   // FP32: uniform spacing, the weights of the first node
+    C ux0[7], ux2[7], uy0[7], uy2[7];   // FP32: the weights of every node
     int macros_on, mass_on;
+
+    // Order of the sums. FP64 filters 7, 8, 9, 10 in y, then x, then xi, and every population with a
+    // y and a xi axis in y first: the least work. FP32 (GATHER) adds the terms in the gather kernel's order
+    // (x, y, xi; 3 and 4 xi, then y) and gives the same bits as that kernel. At nodes where a velocity component
+    // is near zero another order moved it by up to 2.6e-3 of itself (2e-5 is a run's bound).
+    static constexpr bool GATHER = sizeof(C) == 4;
 
     // value of population q at a byte offset (chunk_supported: 32 bits), by a plain load (grid_dependency_wait).
     // 64-bit addresses, one per load, were 40% of the kernel's instructions (FP32 187x91x131 224 us per step).
@@ -71,7 +100,8 @@ struct Chunk {
     static constexpr unsigned EB = sizeof(S);
 
     // Lagrange weights. FP64 takes each node's own: they differ from the first node's by the rounding
-    // of the node positions (about 1e-14), which the 1e-12 parity over a thousand steps would see
+    // of the node positions (about 1e-14), which the 1e-12 parity over a thousand steps would see. FP32
+    // takes the first node's from constant memory (make_chunk_const: equal for all nodes in FP32)
     __device__ __forceinline__ C wx0(int a, int x) const { if constexpr (sizeof(C) == 8) return __ldg(T.wx0 + (size_t)a*k.NX + x); else return ux0[a]; }
     __device__ __forceinline__ C wx2(int a, int x) const { if constexpr (sizeof(C) == 8) return __ldg(T.wx2 + (size_t)a*k.NX + x); else return ux2[a]; }
     __device__ __forceinline__ C wy0(int b, int y) const { if constexpr (sizeof(C) == 8) return __ldg(T.wy0 + (size_t)b*k.NY + y); else return uy0[b]; }
@@ -87,7 +117,7 @@ struct Chunk {
         return v >= NX ? v - NX : v;
     }
 
-    // phase A: y filter of 7, 8, 9, 10 on planes p0 .. p0 + np - 1, columns x0 - 3 .. x0 + W + 2
+    // phase A, FP64: y filter of 7, 8, 9, 10 on planes p0 .. p0 + np - 1, columns x0 - 3 .. x0 + W + 2
     __device__ __forceinline__ void halo_quads(Quad<C> *qb, int p0, int np, int x0, int y0) const {
         const int WH = cc.W + 6, HW = cc.H*WH, NX = k.NX, NY = k.NY;
         for (int i = threadIdx.x; i < np*HW; i += NT) {
@@ -111,52 +141,135 @@ struct Chunk {
 
     struct Col {
         int x, y, xl, yl;
-        bool on;
-        unsigned xo[7];      // byte offsets within a plane: the spanwise stencil's nodes
+        bool on, row;        // a column of the tile; phase A of FP32: a column of the grid
+        unsigned ro, xo[7];  // byte offsets within a plane: the row and, in a row, the spanwise stencil's nodes
         unsigned yo[7];      // and the streamwise stencil's
     };
+    // phase A, FP32: x filter of 7, 8, 9, 10 on planes p0 .. p0 + np - 1, rows y0 - 3 .. y0 + H + 2
+    __device__ __forceinline__ void halo_rows(Quad<C> *qb, int p0, int np, int y0, const Col &L, int g) const {
+        const int RH = cc.H + 6, NX = k.NX, NY = k.NY, per = P/cc.W;
+        if (!L.row) return;
+        for (int line = g*per + L.yl; line < np*RH; line += GROUPS*per) {
+            const int pl = (int)__umulhi((unsigned)line, cc.inv_hw), y = y0 + line - pl*RH - 3;
+            if (y > NY + 2) continue;
+            const unsigned b = (unsigned)(((p0 + pl)*NY + wrap_near(y, NY))*NX)*EB;
+            Sum<C> s7, s8, s9, s10;
+#pragma unroll
+            for (int a = 0; a < 7; a++) {
+                const unsigned o = b + L.xo[a];
+                s7.add(a, wx0(a, L.x), val(7, o));
+                s8.add(a, wx2(a, L.x), val(8, o));
+                s9.add(a, wx0(a, L.x), val(9, o));
+                s10.add(a, wx2(a, L.x), val(10, o));
+            }
+            qb[line*cc.W + L.xl] = Quad<C>{s7.s, s8.s, s9.s, s10.s};
+        }
+    }
 
-    // phase B: ring values of one column on one plane; ring order 3, 4, 5, 6 | 7, 8, 9, 10 |
-    // 11, 12, 13, 14 | 15, 16, 17, 18
+    // phase B: ring values of one column on one plane; ring order 3, 4, 5, 6 (FP32: 5, 6) |
+    // 7, 8, 9, 10 | 11, 12, 13, 14 | 15, 16, 17, 18. qrow: the column's first quad of the plane
     __device__ __forceinline__ void filter(const Col &L, const Quad<C> *qrow, int p, Quad<C> *slot) const {
         const unsigned pl = (unsigned)(p*k.NY*k.NX)*EB;
+        Sum<C> q[4];
         {
-            Quad<C> g{0, 0, 0, 0}, h{0, 0, 0, 0};
+            Sum<C> g[2], h[4];
 #pragma unroll
             for (int j = 0; j < 7; j++) {
                 const unsigned o = pl + L.yo[j];
                 const C w0 = wy0(j, L.y), w2 = wy2(j, L.y);
-                g.a += w0*val(3, o);
-                g.b += w2*val(4, o);
-                h.a += w0*val(15, o);
-                h.b += w2*val(16, o);
-                h.c += w0*val(17, o);
-                h.d += w2*val(18, o);
+                if constexpr (GATHER) {
+                    const Quad<C> v = qrow[j*cc.W];
+                    q[0].add(j, w0, v.a);
+                    q[1].add(j, w0, v.b);
+                    q[2].add(j, w2, v.c);
+                    q[3].add(j, w2, v.d);
+                } else {
+                    g[0].add(j, w0, val(3, o));
+                    g[1].add(j, w2, val(4, o));
+                }
+                h[0].add(j, w0, val(15, o));
+                h[1].add(j, w2, val(16, o));
+                h[2].add(j, w0, val(17, o));
+                h[3].add(j, w2, val(18, o));
             }
-            g.c = val(5, pl + L.yo[3]);
-            g.d = val(6, pl + L.yo[3]);
-            slot[0*P] = g;
-            slot[3*P] = h;
+            slot[0*P] = Quad<C>{g[0].s, g[1].s, val(5, pl + L.yo[3]), val(6, pl + L.yo[3])};
+            slot[3*P] = Quad<C>{h[0].s, h[1].s, h[2].s, h[3].s};
         }
         {
-            Quad<C> g{0, 0, 0, 0}, h{0, 0, 0, 0};
+            Sum<C> h[4];
 #pragma unroll
             for (int a = 0; a < 7; a++) {
-                const unsigned o = pl + L.xo[a];
+                const unsigned o = pl + L.ro + L.xo[a];
                 const C w0 = wx0(a, L.x), w2 = wx2(a, L.x);
-                h.a += w0*val(11, o);
-                h.b += w2*val(12, o);
-                h.c += w0*val(13, o);
-                h.d += w2*val(14, o);
-                const Quad<C> v = qrow[a];
-                g.a += w0*v.a;
-                g.b += w2*v.b;
-                g.c += w0*v.c;
-                g.d += w2*v.d;
+                h[0].add(a, w0, val(11, o));
+                h[1].add(a, w2, val(12, o));
+                h[2].add(a, w0, val(13, o));
+                h[3].add(a, w2, val(14, o));
+                if constexpr (!GATHER) {
+                    const Quad<C> v = qrow[a];
+                    q[0].add(a, w0, v.a);
+                    q[1].add(a, w2, v.b);
+                    q[2].add(a, w0, v.c);
+                    q[3].add(a, w2, v.d);
+                }
             }
-            slot[1*P] = g;
-            slot[2*P] = h;
+            slot[1*P] = Quad<C>{q[0].s, q[1].s, q[2].s, q[3].s};
+            slot[2*P] = Quad<C>{h[0].s, h[1].s, h[2].s, h[3].s};
         }
+    }
+
+    // phase B, FP32: 3 and 4 of targets t0 .. t1 - 1 (at most CHUNK), xi inside y. A warp takes one of the two
+    // populations for half of the targets; four targets read the 10 planes of their windows once.
+    // f34[(t - t0)*2 + population][lane]
+    __device__ __forceinline__ void y_of_xi(const Col &L, int t0, int t1, int g, C *f34) const {
+        static_assert(GROUPS == 4 && CHUNK == 8, "two halves of four targets, two populations");
+        const int pop = g & 1, first = t0 + 4*(g >> 1), last = min(first + 4, t1);
+        const unsigned plane = (unsigned)(k.NY*k.NX)*EB;
+        const S *f = pop ? fq[4] : fq[3];
+        auto xiw = [&](int t, int c) -> C { return __ldg(T.wxi + ((size_t)t*k.NY + L.y)*64 + c*8 + pop); };
+        auto at = [&](unsigned off) -> C { return to_c(*(const S *)((const char *)f + off)); };
+        C *out = f34 + ((first - t0)*2 + pop)*P;
+        if (last - first == 4 && base(last - 1) == base(first) + 3) {
+            C w[4][7];
+            Sum<C> o[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int c = 0; c < 7; c++) w[i][c] = xiw(first + i, c);
+#pragma unroll
+            for (int b = 0; b < 7; b++) {
+                const unsigned off = (unsigned)base(first)*plane + yo_at(L, b);
+                const C wb = pop ? uy2[b] : uy0[b];
+                C v[10];
+#pragma unroll
+                for (int p = 0; p < 10; p++) v[p] = at(off + (unsigned)p*plane);
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    Sum<C> in;
+#pragma unroll
+                    for (int c = 0; c < 7; c++) in.add(c, w[i][c], v[i + c]);
+                    o[i].add(b, wb, in.s);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) out[2*i*P] = o[i].s;
+            return;
+        }
+        for (int t = first; t < last; t++, out += 2*P) {   // windows held at a wall, or fewer targets
+            Sum<C> o;
+#pragma unroll 1
+            for (int b = 0; b < 7; b++) {
+                const unsigned off = (unsigned)base(t)*plane + yo_at(L, b);
+                Sum<C> in;
+#pragma unroll
+                for (int c = 0; c < 7; c++) in.add(c, xiw(t, c), at(off + (unsigned)c*plane));
+                o.add(b, pop ? uy2[b] : uy0[b], in.s);
+            }
+            *out = o.s;
+        }
+    }
+    __device__ __forceinline__ unsigned yo_at(const Col &L, int b) const {
+        return (unsigned)(wrap_near(L.y - 3 + b, k.NY)*k.NX + L.x)*EB;
     }
 
     // BFL rows: which sums a flagged row needs. Kinds 0..3 (with the halo columns): 7, 8, 9, 10 from
@@ -164,6 +277,7 @@ struct Chunk {
     // and weight sets (C/evolution.h:505-572).
     __device__ __forceinline__ static int kind_flag(int kd) { return kd < 2 ? 0 : kd < 4 ? 1 : kd - 4; }
     __device__ __forceinline__ static int kind_src(int kd) { return kd < 4 ? 10 - kd : kd == 4 ? 4 : kd == 5 ? 3 : kd == 6 ? 18 : 17; }
+    __device__ __forceinline__ static int kind_xset(int kd) { return kd == 0 ? B_XB37 : kd == 1 ? B_XB38 : kd == 2 ? B_XB49 : B_XB410; }
     __device__ __forceinline__ static int kind_yset(int fl) { return fl == 0 ? B_YB378 : fl == 1 ? B_YB4910 : fl == 2 ? B_YB15 : B_YB16; }
     __device__ __forceinline__ static int kind_zset(int fl) { return fl == 0 ? B_XIB378 : fl == 1 ? B_XIB4910 : fl == 2 ? B_XIB15 : B_XIB16; }
 
@@ -172,13 +286,14 @@ struct Chunk {
         return idx < nb ? __ldg(T.bfl_w + ((size_t)s*7 + a)*nb + idx) : C(0);
     }
 
-    // (y, xi) sums of the flagged rows z = z0 .. z1 - 1 of the tile:
-    // bf[((z*H + yl)*8 + kind)*(W + 6) + xx]. The flagged (row, kind) pairs are listed first, so that
-    // all of them are summed in one pass of the CTA (row after row, their load latencies add up).
+    // Sums of the flagged rows z = z0 .. z1 - 1 of the tile, bf[((z*H + yl)*8 + kind)*per + xx]. FP64: the (y, xi)
+    // sums with the halo columns (per = W + 6); FP32: the whole sums (per = W). The flagged (row, kind)
+    // pairs are listed first, so that all of them are summed in one pass of the CTA (row after row, their
+    // load latencies add up).
     __device__ __forceinline__ void bfl_sums(C *bf, int z0, int z1, int x0, int y0) const {
         __shared__ int count;
         __shared__ unsigned short list[2*P*8];
-        const int WH = cc.W + 6, NX = k.NX, NY = k.NY, nb = 2*k.NYD6;
+        const int NX = k.NX, NY = k.NY, nb = 2*k.NYD6;
         if (threadIdx.x == 0) count = 0;
         __syncthreads();
         for (int i = z0*cc.H*8 + threadIdx.x; i < z1*cc.H*8; i += NT) {
@@ -186,45 +301,69 @@ struct Chunk {
             if (y < NY && T.bfl_flag[fl*nb + r] == 1 && T.bfl_q[fl*nb + r] < C(0.5)) list[atomicAdd(&count, 1)] = (unsigned short)i;
         }
         __syncthreads();
-        const int items = count*WH;
+        const int per = GATHER ? cc.W : cc.W + 6, items = count*per;
         for (int i = threadIdx.x; i < items; i += NT) {
-            const int e = list[i/WH], xx = i % WH, kd = e & 7, fl = kind_flag(kd), q = kind_src(kd);
+            const int m = i/per, xx = i - m*per, e = list[m], kd = e & 7, fl = kind_flag(kd), q = kind_src(kd);
             const int z = e/(8*cc.H), y = y0 + (e/8) % cc.H, r = z*k.NYD6 + y + 3;
             const int iy = k.bfl_mode ? r : y + 3;   // reference: Y weights at [j]
-            const unsigned b = (unsigned)wrap_x(x0 + xx - 3);
+            if (GATHER && x0 + xx >= NX) continue;
+            const unsigned b = (unsigned)(GATHER ? x0 + xx : wrap_x(x0 + xx - 3));
             const S *f = fq[q];
             C wy[7], sum = 0;
 #pragma unroll
             for (int j = 0; j < 7; j++) wy[j] = bw(kind_yset(fl), j, iy);
+            if (GATHER && kd < 4) {
+                const int x = x0 + xx, ix = k.bfl_mode ? r : x + 3;
+                C wx[7];
+                unsigned xo[7];
 #pragma unroll
-            for (int c = 0; c < 7; c++) {
-                C in = 0;
+                for (int a = 0; a < 7; a++) { wx[a] = bw(kind_xset(kd), a, ix); xo[a] = (unsigned)wrap_any(x - 3 + a, NX); }
+#pragma unroll 1
+                for (int c = 0; c < 7; c++) {
+                    C mid = 0;
 #pragma unroll
-                for (int j = 0; j < 7; j++) {
-                    in += to_c(f[b + (unsigned)((c*NY + wrap_near(y - 3 + j, NY))*NX)])*wy[j];
+                    for (int j = 0; j < 7; j++) {
+                        const unsigned row = (unsigned)((c*NY + wrap_near(y - 3 + j, NY))*NX);
+                        C in = 0;
+#pragma unroll
+                        for (int a = 0; a < 7; a++) in += to_c(f[row + xo[a]])*wx[a];
+                        mid += in*wy[j];
+                    }
+                    sum += mid*bw(kind_zset(fl), c, r);
                 }
-                sum += in*bw(kind_zset(fl), c, r);
+            } else {
+#pragma unroll
+                for (int c = 0; c < 7; c++) {
+                    C in = 0;
+#pragma unroll
+                    for (int j = 0; j < 7; j++) in += to_c(f[b + (unsigned)((c*NY + wrap_near(y - 3 + j, NY))*NX)])*wy[j];
+                    sum += in*bw(kind_zset(fl), c, r);
+                }
             }
-            bf[(size_t)e*WH + xx] = sum;
+            bf[(size_t)e*per + xx] = sum;
         }
     }
 
     __device__ __forceinline__ void bfl_apply(C (&F)[19], const Col &L, int z, const C *bf) const {
-        const int NX = k.NX, NY = k.NY, nb = 2*k.NYD6, WH = cc.W + 6;
+        const int NX = k.NX, NY = k.NY, nb = 2*k.NYD6;
         const int r = z*k.NYD6 + L.y + 3;
         const int ix = k.bfl_mode ? r : L.x + 3;   // reference: X weights at [i]
         const unsigned nd = (unsigned)((z*NY + L.y)*NX + L.x)*EB;
+        const int WH = GATHER ? cc.W : cc.W + 6;   // values of a kind
         const C *row = bf + (size_t)(z*cc.H + L.yl)*8*WH + L.xl;
         auto lin = [&](C q, int a, int b) -> C {   // (1/(2Q)) f_a + ((2Q-1)/(2Q)) f_b at the node
             return (C(1)/(C(2)*q))*val(a, nd) + ((C(2)*q - C(1))/(C(2)*q))*val(b, nd);
         };
+        auto at = [&](int kd) -> C {
+            return row[kd*WH + (GATHER ? 0 : 3)];
+        };
         auto xf = [&](int kd, int set) -> C {
+            if constexpr (GATHER) return at(kd);
             C s = 0;
 #pragma unroll
             for (int a = 0; a < 7; a++) s += bw(set, a, ix)*row[kd*WH + a];
             return s;
         };
-        auto at = [&](int kd) -> C { return row[kd*WH + 3]; };
         if (T.bfl_flag[0*nb + r] == 1) {
             const C q = T.bfl_q[0*nb + r];
             if (q > C(0.5)) { F[3] = lin(q, 4, 3); F[7] = lin(q, 10, 7); F[8] = lin(q, 9, 8); }
@@ -248,15 +387,14 @@ struct Chunk {
     }
 
     // phase C: target plane t of one column
-    __device__ __forceinline__ void target(const Col &L, const Quad<C> *ring, int t, const C *bf, C f6, C f12, C rho_mod,
+    // (f34: FP32, the sums of y_of_xi for this target)
+    __device__ __forceinline__ void target(const Col &L, const Quad<C> *ring, int t, const C *f34, const C *bf, C f6, C f12, C rho_mod,
                                            double &ub, double &mass) const {
         const int NX = k.NX, NY = k.NY;
         const int b = base(t);
         C F[19];
         {
-            C a[16];
-#pragma unroll
-            for (int j = 0; j < 16; j++) a[j] = 0;
+            Sum<C> a[16];
             const Quad<C> *w = (const Quad<C> *)(T.wxi + ((size_t)t*NY + L.y)*64);
             int slot = b % RING;
 #pragma unroll
@@ -264,22 +402,29 @@ struct Chunk {
                 const Quad<C> w0 = w[2*c], w1 = w[2*c + 1];   // xi 3, 4, 5, 6 | 15, 16, 17, 18
                 const Quad<C> *v = ring + (size_t)slot*4*P;
                 const Quad<C> v0 = v[0], v1 = v[P], v2 = v[2*P], v3 = v[3*P];
-                a[0] += w0.a*v0.a; a[1] += w0.b*v0.b; a[2] += w0.c*v0.c; a[3] += w0.d*v0.d;
-                a[4] += w0.a*v1.a; a[5] += w0.a*v1.b; a[6] += w0.b*v1.c; a[7] += w0.b*v1.d;
-                a[8] += w0.c*v2.a; a[9] += w0.c*v2.b; a[10] += w0.d*v2.c; a[11] += w0.d*v2.d;
-                a[12] += w1.a*v3.a; a[13] += w1.b*v3.b; a[14] += w1.c*v3.c; a[15] += w1.d*v3.d;
+                if constexpr (!GATHER) { a[0].add(c, w0.a, v0.a); a[1].add(c, w0.b, v0.b); }
+                a[2].add(c, w0.c, v0.c); a[3].add(c, w0.d, v0.d);
+                const C m7[4] = {w0.a, w0.a, w0.b, w0.b}, f7[4] = {v1.a, v1.b, v1.c, v1.d};
+#pragma unroll
+                for (int m = 0; m < 4; m++) {   // (the gather kernel's loop over these is not unrolled)
+                    if constexpr (GATHER) a[4 + m].s = __fmaf_rn(m7[m], f7[m], a[4 + m].s);
+                    else a[4 + m].add(c, m7[m], f7[m]);
+                }
+                a[8].add(c, w0.c, v2.a); a[9].add(c, w0.c, v2.b); a[10].add(c, w0.d, v2.c); a[11].add(c, w0.d, v2.d);
+                a[12].add(c, w1.a, v3.a); a[13].add(c, w1.b, v3.b); a[14].add(c, w1.c, v3.c); a[15].add(c, w1.d, v3.d);
                 slot = slot == RING - 1 ? 0 : slot + 1;
             }
 #pragma unroll
-            for (int j = 0; j < 16; j++) F[3 + j] = a[j];
+            for (int j = 0; j < 16; j++) F[3 + j] = a[j].s;
+            if constexpr (GATHER) { F[3] = f34[0]; F[4] = f34[P]; }
         }
         const unsigned node = (unsigned)((t*NY + L.y)*NX + L.x), nd = node*EB;
         {
-            const unsigned pl = (unsigned)(t*NY*NX)*EB;
-            C s1 = 0, s2 = 0;
+            const unsigned row = (unsigned)(t*NY*NX)*EB + L.ro;
+            Sum<C> s1, s2;
 #pragma unroll
-            for (int a = 0; a < 7; a++) { s1 += wx0(a, L.x)*val(1, pl + L.xo[a]); s2 += wx2(a, L.x)*val(2, pl + L.xo[a]); }
-            F[1] = s1; F[2] = s2;
+            for (int a = 0; a < 7; a++) { s1.add(a, wx0(a, L.x), val(1, row + L.xo[a])); s2.add(a, wx2(a, L.x), val(2, row + L.xo[a])); }
+            F[1] = s1.s; F[2] = s2.s;
             F[0] = val(0, nd);
         }
         auto opp = [&](int q) -> C { return val(q, nd); };
@@ -299,9 +444,10 @@ struct Chunk {
 
     __device__ __forceinline__ void run(unsigned char *smem) const {
         Quad<C> *ring = (Quad<C> *)smem;
-        Quad<C> *qb = (Quad<C> *)(smem + ring_bytes<C>());
+        C *f34 = (C *)(smem + ring_bytes<C>());
+        Quad<C> *qb = (Quad<C> *)(smem + ring_bytes<C>() + f34_bytes<C>());
         const int tid = threadIdx.x, c = tid % P, g = tid/P;
-        const int WH = cc.W + 6, NX = k.NX, NY = k.NY, NZ = k.NZ;
+        const int NX = k.NX, NY = k.NY, NZ = k.NZ;
         double ub = 0.0, mass = 0.0;
         const double force = ctrl->force;
         const C f6 = (C)(1.0/6*force*k.dt), f12 = (C)(1.0/12*force*k.dt), rho_mod = (C)ctrl->rho_modify;
@@ -314,10 +460,12 @@ struct Chunk {
             L.yl = c/cc.W; L.xl = c - L.yl*cc.W;
             L.x = x0 + L.xl; L.y = y0 + L.yl;
             L.on = L.yl < cc.H && L.x < NX && L.y < NY;
-            if (L.on) {
+            L.row = L.yl < P/cc.W && L.x < NX;
+            L.ro = (unsigned)(L.y*NX)*EB;
+            if (GATHER ? L.row : L.on) {
 #pragma unroll
                 for (int a = 0; a < 7; a++) {
-                    L.xo[a] = (unsigned)(L.y*NX + wrap_any(L.x - 3 + a, NX))*EB;
+                    L.xo[a] = (unsigned)wrap_any(L.x - 3 + a, NX)*EB;
                     L.yo[a] = (unsigned)(wrap_near(L.y - 3 + a, NY)*NX + L.x)*EB;
                 }
             }
@@ -325,12 +473,20 @@ struct Chunk {
             for (int t0 = ta; t0 < tb; t0 += CHUNK) {
                 const int t1 = min(t0 + CHUNK, tb);
                 const int pend = base(t1 - 1) + 7;
-                halo_quads(qb, np, pend - np, x0, y0);
-                __syncthreads();   // quads complete; every thread is done with the previous chunk's targets
-                if (L.on)
-                    for (int p = np + g; p < pend; p += GROUPS)
-                        filter(L, qb + (size_t)((p - np)*cc.H + L.yl)*WH + L.xl, p, ring + (size_t)(p % RING)*4*P + c);
-                np = pend;
+                while (true) {
+                    const int pb = min(np + batch<C>(), pend);
+                    if constexpr (GATHER) halo_rows(qb, np, pb - np, y0, L, g);
+                    else halo_quads(qb, np, pb - np, x0, y0);
+                    __syncthreads();   // quads complete; every thread is done with the previous chunk's targets
+                    if (L.on)
+                        for (int p = np + g; p < pb; p += GROUPS)
+                            filter(L, qb + (GATHER ? ((p - np)*(cc.H + 6) + L.yl)*cc.W : ((p - np)*cc.H + L.yl)*(cc.W + 6)) + L.xl, p,
+                                   ring + (size_t)(p % RING)*4*P + c);
+                    np = pb;
+                    if (np >= pend) break;
+                    __syncthreads();   // quads free
+                }
+                if constexpr (GATHER) { if (L.on) y_of_xi(L, t0, t1, g, f34 + c); }
                 __syncthreads();   // ring complete, quads free
                 if (t0 <= 1) {
                     bfl_sums((C *)qb, t0, min(t1, 2), x0, y0);
@@ -338,7 +494,7 @@ struct Chunk {
                 }
                 if (L.on)
                     for (int t = t0 + g; t < t1; t += GROUPS)
-                        target(L, ring + c, t, (const C *)qb, f6, f12, rho_mod, ub, mass);
+                        target(L, ring + c, t, f34 + (t - t0)*2*P + c, (const C *)qb, f6, f12, rho_mod, ub, mass);
                 if (t0 <= 1) __syncthreads();   // the sums are read before the next chunk's quads replace them
             }
         }
@@ -346,12 +502,12 @@ struct Chunk {
     }
 };
 
-// CTAs per SM: shared memory (ring + quads) allows 3 in FP64 (about 71 KB) and 6 in FP32; registers
-// 168 and 128 per thread without spills
-template <class S> constexpr int min_ctas() { return sizeof(typename Storage<S>::C) == 8 ? 3 : 4; }
+// CTAs per SM: shared memory (ring + quads) allows 3 in FP64 (about 71 KB) and 2 in FP32 (81 KB at 16x4);
+// 168 registers per thread in FP64 and 128 in FP32
+template <class S> constexpr int min_ctas() { return sizeof(typename Storage<S>::C) == 8 ? 3 : 2; }
 
 template <class S, bool LES>
-__global__ void __launch_bounds__(NT, min_ctas<S>()) step_chunk_kernel(const __grid_constant__ Chunk<S, LES> K) {
+__global__ void __launch_bounds__(Chunk<S, LES>::NT, min_ctas<S>()) step_chunk_kernel(const __grid_constant__ Chunk<S, LES> K) {
     extern __shared__ __align__(128) unsigned char smem[];
     // the trigger comes after the wait: at most two steps are resident at a time
     grid_dependency_wait();
@@ -360,15 +516,17 @@ __global__ void __launch_bounds__(NT, min_ctas<S>()) step_chunk_kernel(const __g
 }
 
 template <class C> size_t smem_for(int W, int H) {
-    const size_t quads = (size_t)RING*H*(W + 6)*sizeof(Quad<C>), sums = (size_t)2*H*8*(W + 6)*sizeof(C);
-    return ring_bytes<C>() + std::max(quads, sums);
+    const bool rows = sizeof(C) == 4;   // halo rows (FP32) or halo columns
+    const size_t quads = (size_t)batch<C>()*(rows ? (H + 6)*W : H*(W + 6))*sizeof(Quad<C>);
+    const size_t sums = (size_t)2*H*8*(rows ? W : W + 6)*sizeof(C);
+    return ring_bytes<C>() + f34_bytes<C>() + std::max(quads, sums);
 }
 
 template <class S, bool LES>
 cudaError_t prepare_t(size_t smem, int *ctas) {
     cudaError_t e = cudaFuncSetAttribute(step_chunk_kernel<S, LES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas, step_chunk_kernel<S, LES>, NT, smem);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas, step_chunk_kernel<S, LES>, Chunk<S, LES>::NT, smem);
 }
 
 template <class S, bool LES>
@@ -388,7 +546,7 @@ cudaError_t launch_t(const StepLaunch &L) {
         K.uy0[a] = (C)K.cc.wy0[a]; K.uy2[a] = (C)K.cc.wy2[a];
     }
     K.macros_on = L.macros_on; K.mass_on = L.mass;
-    return launch_dependent(step_chunk_kernel<S, LES>, K.cc.grid, NT, K.cc.smem_bytes, L.stream, K);
+    return launch_dependent(step_chunk_kernel<S, LES>, K.cc.grid, Chunk<S, LES>::NT, K.cc.smem_bytes, L.stream, K);
 }
 
 template <class F>
@@ -412,18 +570,42 @@ cudaError_t make_chunk_const(const StepConst &k, int precision, bool les, const 
     ChunkConst cc;
     std::memset((void *)&cc, 0, sizeof(cc));
     for (int a = 0; a < 7; a++) { cc.wx0[a] = wx0[a]; cc.wx2[a] = wx2[a]; cc.wy0[a] = wy0[a]; cc.wy2[a] = wy2[a]; }
-    // tile shape: the split of a row into equal parts of at most 32 columns, H rows of it, with the
-    // fewest warps per node; a part costs 32 lanes in phases B and C (about 0.95 of the work)
-    // and its halo columns in phase A
+    const bool rows = precision != ISLBM_FP64;   // phase A takes halo rows (FP32) or halo columns
+    const int P = rows ? lanes<float>() : lanes<double>();
+    // wall-normal segments: rounds of items x (targets per segment + the ramp of 6 planes, whose
+    // filters cost a quarter of a whole plane in FP64 and about half in FP32), down to one target
+    // where a grid has few tiles
+    const double ramp = precision == ISLBM_FP64 ? 1.5 : 3.0;
+    auto makespan = [&](int tiles, int slots, int &segs) {
+        double best = 1e300;
+        for (int z = 1; z <= k.NZ; z++) {
+            const long long items = (long long)tiles*z;
+            const double rounds = (double)((items + slots - 1)/slots);
+            const double cost = rounds*((double)((k.NZ + z - 1)/z) + ramp);
+            if (cost < best - 1e-9) { best = cost; segs = z; }
+        }
+        return best;
+    };
+    // tile shape: a split of a row into equal parts of at most P columns, H rows of it. FP64: the fewest warps
+    // per node; a part costs 32 lanes in phases B and C (about 0.95 of the work) and its halo columns
+    // in phase A. FP32: the shortest makespan; a plane of a tile costs 1 + 0.0038 per halo-row value + 0.089
+    // per row (the more rows, the shorter the runs of addresses): 187x91x131 in one round of 304 CTAs
+    // 16x4 262 us per step, 12x5 272, 31x2 283, 8x8 285, and 13x4, which takes a second round, 350
     double best = 1e300;
     for (int parts = (k.NX + P - 1)/P; parts <= k.NX; parts++) {
         const int W = (k.NX + parts - 1)/parts, tx = (k.NX + W - 1)/W;
         const int H = std::min(P/W, k.NY), ty = (k.NY + H - 1)/H;
-        const double cost = (double)tx*ty*(0.95*P + 0.05*H*(W + 6));
+        double cost = (double)tx*ty*(0.95*P + 0.05*H*(W + 6));
+        if (rows) {
+            const int fit = (int)(228*1024/(smem_for<float>(W, H) + 4096));
+            int z;
+            cost = makespan(tx*ty, std::max(1, std::min(fit, min_ctas<float>()))*num_sms, z)*(1.0 + 0.0038*(H + 6)*W + 0.089*H);
+        }
         if (cost < best*(1.0 - 1e-9)) { best = cost; cc.W = W; cc.H = H; cc.tiles_x = tx; cc.tiles_y = ty; }
         if (W <= 4) break;
     }
-    cc.inv_hw = (unsigned)((0x100000000ULL + cc.H*(cc.W + 6) - 1)/(cc.H*(cc.W + 6)));
+    const unsigned per_plane = (unsigned)(rows ? cc.H + 6 : cc.H*(cc.W + 6));
+    cc.inv_hw = (unsigned)((0x100000000ULL + per_plane - 1)/per_plane);
     cc.inv_wh = (unsigned)((0x100000000ULL + cc.W + 5)/(cc.W + 6));
     cc.smem_bytes = precision == ISLBM_FP64 ? smem_for<double>(cc.W, cc.H) : smem_for<float>(cc.W, cc.H);
     int ctas = 0;
@@ -433,18 +615,8 @@ cudaError_t make_chunk_const(const StepConst &k, int precision, bool les, const 
     });
     if (e != cudaSuccess) return e;
     if (ctas < 1) return cudaErrorInvalidConfiguration;
-    // wall-normal segments: rounds of items x (targets per segment + the ramp of 6 planes, whose
-    // filters cost a quarter of a whole plane in FP64 and about half in FP32), down to one target
-    // where a grid has few tiles
     const int tiles = cc.tiles_x*cc.tiles_y, slots = ctas*num_sms;
-    const double ramp = precision == ISLBM_FP64 ? 1.5 : 3.0;
-    double best_cost = 1e300;
-    for (int z = 1; z <= k.NZ; z++) {
-        const long long items = (long long)tiles*z;
-        const double rounds = (double)((items + slots - 1)/slots);
-        const double cost = rounds*((double)((k.NZ + z - 1)/z) + ramp);
-        if (cost < best_cost - 1e-9) { best_cost = cost; cc.segs = z; }
-    }
+    makespan(tiles, slots, cc.segs);
     cc.grid = (int)std::min<long long>((long long)tiles*cc.segs, slots);
     *out = cc;
     return cudaSuccess;

@@ -15,7 +15,7 @@ struct ChunkConst {
     int tiles_x, tiles_y;
     int segs;                  // wall-normal segments per column
     int grid;                  // persistent CTAs
-    unsigned inv_hw, inv_wh;   // 2^32/(H*(W + 6)) and 2^32/(W + 6), rounded up: exact quotients by __umulhi
+    unsigned inv_hw, inv_wh;   // 2^32/(H*(W + 6)) (FP32: H + 6) and 2^32/(W + 6), rounded up: exact quotients by __umulhi
     size_t smem_bytes;
     double wx0[7], wx2[7], wy0[7], wy2[7];   // uniform-spacing Lagrange weights
 };

@@ -492,12 +492,10 @@ int init_impl(const islbm_params *pp, islbm_handle *h) {
         // for (comparison runs)
         const char *cp = std::getenv("ISLBM_PAIR_COPIES");
         const bool maps = !(cp && std::strcmp(cp, "bulk") == 0);
-        // (a tiled kernel asked for by name stays refused on the grids whose rows do not divide into tiles)
-        const bool named = p.kernel == ISLBM_KERNEL_TILED && !pair_supported(k, p.precision) && !tiled_supported(k, p.precision);
-        // 16-bit storage amplifies every change of rounding: those grids keep the arithmetic of the kernels
-        // they have had (the role kernel's is the paired one's, bit for bit)
-        const bool same = p.precision == ISLBM_FP32 || pair_supported(k, p.precision);
-        if (p.kernel != ISLBM_KERNEL_TILED_SINGLE && !named && same && roles_supported(k, p.precision)) {
+        // (the role kernel gives the paired one's bits and replaces it only: grids whose rows the paired
+        // kernel does not divide keep the one-node-per-thread kernel's results, or the gather kernel's,
+        // whose sums are in another order)
+        if (p.kernel != ISLBM_KERNEL_TILED_SINGLE && pair_supported(k, p.precision) && roles_supported(k, p.precision)) {
             CK(make_roles_const(k, p.precision, p.les_cs > 0.0, wx0, wx2, wy0, wy2, sms, &h->tiled));
             h->use_tiled = h->paired = h->roles = true;
             if (maps) make_role_maps(k, (int)h->elem, h->fbuf, &h->rmaps);

@@ -24,6 +24,10 @@ ISLBM_API int islbm_fault_drill(islbm_handle *h, int plane);
 enum { ISLBM_STEP_GATHER = 0, ISLBM_STEP_CHUNK = 1, ISLBM_STEP_TILED = 2, ISLBM_STEP_PAIRED = 3, ISLBM_STEP_ROLES = 4 };
 ISLBM_API int islbm_step_kernel(const islbm_handle *h, int *kernel);
 
+/* From the next islbm_step on, a solve that steps with the role-specialised kernel steps with the
+ * paired one, whose results are the same bits (runs that compare the two). */
+ISLBM_API int islbm_use_paired(islbm_handle *h);
+
 #ifdef __cplusplus
 }
 #endif

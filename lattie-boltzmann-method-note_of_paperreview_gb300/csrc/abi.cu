@@ -413,6 +413,20 @@ void free_handle_impl(islbm_handle *h) {
     delete h;
 }
 
+// uniform spacing: the weights of the first node serve all
+void first_weights(const Geometry &g, double (&wx0)[7], double (&wx2)[7], double (&wy0)[7], double (&wy2)[7]) {
+    for (int a = 0; a < 7; a++) {
+        wx0[a] = g.XP0[(size_t)a*g.NX6 + 3]; wx2[a] = g.XP2[(size_t)a*g.NX6 + 3];
+        wy0[a] = g.YP0[(size_t)a*g.NYD6 + 3]; wy2[a] = g.YP2[(size_t)a*g.NYD6 + 3];
+    }
+}
+
+// tensor-map plane copies unless the bulk row copies are asked for (comparison runs)
+bool map_copies() {
+    const char *cp = std::getenv("ISLBM_PAIR_COPIES");
+    return !(cp && std::strcmp(cp, "bulk") == 0);
+}
+
 int init_impl(const islbm_params *pp, islbm_handle *h) {
     h->p = *pp;
     const int st = h->g.build(*pp);
@@ -482,16 +496,11 @@ int init_impl(const islbm_params *pp, islbm_handle *h) {
     int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
     double wx0[7], wx2[7], wy0[7], wy2[7];
-    for (int a = 0; a < 7; a++) {   // uniform spacing: the weights of the first node serve all
-        wx0[a] = h->g.XP0[(size_t)a*h->g.NX6 + 3]; wx2[a] = h->g.XP2[(size_t)a*h->g.NX6 + 3];
-        wy0[a] = h->g.YP0[(size_t)a*h->g.NYD6 + 3]; wy2[a] = h->g.YP2[(size_t)a*h->g.NYD6 + 3];
-    }
+    first_weights(h->g, wx0, wx2, wy0, wy2);
     if (p.kernel == ISLBM_KERNEL_TILED || p.kernel == ISLBM_KERNEL_AUTO || p.kernel == ISLBM_KERNEL_TILED_SINGLE) {
         // the role-specialised paired kernel where the grid allows it, else the paired one, else the
-        // one-node-per-thread kernel; tensor-map plane copies unless the bulk row copies are asked
-        // for (comparison runs)
-        const char *cp = std::getenv("ISLBM_PAIR_COPIES");
-        const bool maps = !(cp && std::strcmp(cp, "bulk") == 0);
+        // one-node-per-thread kernel
+        const bool maps = map_copies();
         // (the role kernel gives the paired one's bits and replaces it only: grids whose rows the paired
         // kernel does not divide keep the one-node-per-thread kernel's results, or the gather kernel's,
         // whose sums are in another order)
@@ -749,6 +758,23 @@ int islbm_step_kernel(const islbm_handle *h, int *kernel) {
     if (check_handle(h) || !kernel) return ISLBM_ERR_INVALID_ARGUMENT;
     *kernel = h->roles ? ISLBM_STEP_ROLES : h->paired ? ISLBM_STEP_PAIRED : h->use_tiled ? ISLBM_STEP_TILED
             : h->chunked ? ISLBM_STEP_CHUNK : ISLBM_STEP_GATHER;
+    return ISLBM_OK;
+}
+
+int islbm_use_paired(islbm_handle *h) {
+    if (check_handle(h)) return ISLBM_ERR_INVALID_ARGUMENT;
+    if (!h->roles) { g_last = "the solve does not step with the role kernel"; return ISLBM_ERR_NOT_SUPPORTED; }
+    CK(cudaSetDevice(h->device));
+    int sms = 0;
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+    double wx0[7], wx2[7], wy0[7], wy2[7];
+    first_weights(h->g, wx0, wx2, wy0, wy2);
+    TiledConst tc;
+    if (!pair_supported(h->k, h->p.precision) || make_pair_const(h->k, h->p.precision, wx0, wx2, wy0, wy2, sms, &tc) != 0)
+        return ISLBM_ERR_NOT_SUPPORTED;
+    h->tiled = tc;
+    h->roles = false;
+    if (map_copies()) make_pair_maps(h->k, (int)h->elem, h->fbuf, &h->pmaps);
     return ISLBM_OK;
 }
 

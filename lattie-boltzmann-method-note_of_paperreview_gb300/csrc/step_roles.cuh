@@ -52,8 +52,8 @@ template <> struct Regs<float> { static constexpr int collide = 152, rows = 80, 
 constexpr int SLOTS = 8;              // ring planes
 
 // named barriers: 1 collide warps, 2 work item (batched kernel), 3, 4 filter row groups, 5 end of the
-// ring's use (filter warps arrive, collide warps wait), 8.. collide rows
-constexpr int BAR_COLLIDE = 1, BAR_ITEM = 2, BAR_FILTER = 3, BAR_RING_END = 5, BAR_ROW = 8;
+// ring's use (filter warps arrive, collide warps wait)
+constexpr int BAR_COLLIDE = 1, BAR_ITEM = 2, BAR_FILTER = 3, BAR_RING_END = 5;
 constexpr int RING_THREADS = 32*(COLLIDE_WARPS + FILTER_WARPS);
 
 template <int R> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
@@ -82,7 +82,7 @@ __host__ __device__ constexpr int FQ(int i) {
 //   NFS front stages; NTS target stages (populations 0, 1, 2 as TY rows, then the rows' duplicated
 //   xi weights, TY x 128 floats); ybuf [2][TY][2][NX/2] float4: streamwise-filtered (7, 8, 9, 10)
 //   by plane parity, the even and the odd node of each pair apart (consecutive threads, consecutive
-//   16 bytes); bfl [2][512] floats; mbarriers; timeout flag and TMEM address.
+//   16 bytes); mbarriers; timeout flag and TMEM address.
 template <class S, int NXC>
 struct RLay {
     static constexpr int NX = NXC, PR = NX/2, TY = 512/NX;
@@ -96,19 +96,18 @@ struct RLay {
     static constexpr int w_off = up128(3*plain_pop);
     static constexpr int target_bytes = w_off + TY*512;
     static constexpr unsigned target_tx = (unsigned)(3*plain_pop + TY*512);
-    static constexpr int ybuf_bytes = 2*512*16, bfl_bytes = 2*512*4;
+    static constexpr int ybuf_bytes = 2*512*16;
     // front stages: as many as fit, up to three. The copies of a plane take about 2.5 us from issue to
     // completion under load, longer than a plane's work: with two stages the copies' latency set
     // the pace (FP32 256x128x192 without collisions and stores 184 us per step, with them 207)
-    static constexpr int room = 227*1024 - ybuf_bytes - bfl_bytes - 1536;
+    static constexpr int room = 227*1024 - ybuf_bytes - 1536;
     static constexpr int fit = (room - 2*target_bytes)/front_bytes;
     static constexpr int NFS = fit > 3 ? 3 : fit;
     static constexpr int NTS = NFS*front_bytes + 4*target_bytes <= room ? 4 : 2;
     static_assert(NFS >= 2, "two front stages");
     static constexpr int target_off = NFS*front_bytes;
     static constexpr int ybuf_off = target_off + NTS*target_bytes;
-    static constexpr int bfl_off = ybuf_off + ybuf_bytes;
-    static constexpr int bar_off = bfl_off + bfl_bytes;
+    static constexpr int bar_off = ybuf_off + ybuf_bytes;
     // mbarriers: front full, front empty, target full, target empty, ring full and ring free per
     // lane quarter and slot
     static constexpr int B_FF = 0, B_FE = NFS, B_TF = 2*NFS, B_TE = B_TF + NTS, B_RF = B_TE + NTS, B_RE = B_RF + 4*SLOTS;
@@ -471,20 +470,60 @@ struct RoleKernel {
         const int nb = 2*k.NYD6;
         return idx < nb ? __ldg(T.bfl_w + ((size_t)s*7 + a)*nb + idx) : 0.f;
     }
-    __device__ __forceinline__ void row_sync(int row) const {
-        if constexpr (PR > 32) bar_sync(BAR_ROW + row, PR);
-        else __syncwarp(PR == 32 ? 0xffffffffu : (0xffffu << (threadIdx.x & 16)));
+    // Sums of the opposite populations for wall distances below one half, in the order of the paired and
+    // gather kernels (x innermost, then y, then xi): FP16 storage carries a changed last place on, and
+    // 2,000 steps over the steep hill (alpha 0.73, whose first rows are such) made 9e-4 of it. (A
+    // twelve-solve burst on 64x32x48: 187 ms, with the sums in y and xi first, x last, 175.)
+    // y and xi only (populations without an x axis):
+    __device__ __forceinline__ V2 bfl_y_xi(int q, int yset, int zset, int x0, int y, int r, int iy) const {
+        const size_t N = (size_t)NX*k.NY*k.NZ;
+        V2 g = V2(0.f);
+#pragma unroll 1
+        for (int c = 0; c < 7; c++) {
+            V2 in = V2(0.f);
+#pragma unroll
+            for (int b = 0; b < 7; b++) in = V2(bw(yset, b, iy))*ld2g<S>(fo + q*N + bfl_row(c, y - 3 + b) + x0, q) + in;
+            g = V2(bw(zset, c, r))*in + g;
+        }
+        return g;
+    }
+    // x, y and xi: a node pair's stencils are five aligned pairs of every row
+    __device__ __forceinline__ V2 bfl_x_y_xi(int q, int xset, int yset, int zset, int x0, int y, int r, int iy) const {
+        const size_t N = (size_t)NX*k.NY*k.NZ;
+        V2 wx[7], g = V2(0.f);
+#pragma unroll
+        for (int a = 0; a < 7; a++)   // reference: X weights at [i]
+            wx[a] = k.bfl_mode ? V2(bw(xset, a, r)) : V2(bw(xset, a, x0 + 3), bw(xset, a, x0 + 4));
+#pragma unroll 1
+        for (int c = 0; c < 7; c++) {
+            V2 mid = V2(0.f);
+#pragma unroll
+            for (int b = 0; b < 7; b++) {
+                const S *p = fo + q*N + bfl_row(c, y - 3 + b);
+                V2 f[5], in = V2(0.f);
+#pragma unroll
+                for (int m = 0; m < 5; m++) f[m] = ld2g<S>(p + ((x0 - 4 + 2*m) & (NX - 1)), q);
+#pragma unroll
+                for (int a = 0; a < 7; a++)
+                    in = wx[a]*((a & 1) ? f[(a + 1)/2] : V2(f[a/2].v.y, f[a/2 + 1].v.x)) + in;
+                mid = V2(bw(yset, b, iy))*in + mid;
+            }
+            g = V2(bw(zset, c, r))*mid + g;
+        }
+        return g;
+    }
+    __device__ __forceinline__ size_t bfl_row(int c, int yy) const {
+        const int NY = k.NY;
+        yy = yy < 0 ? yy + NY : (yy >= NY ? yy - NY : yy);
+        return ((size_t)c*NY + yy)*NX;
     }
 
-    // One flag type of the BFL rows (C/evolution.h:505-572) of a whole row y at plane z <= 1, called
-    // by the row's threads together. dst / src: populations set and their opposites, the first without
-    // and the other two with an x filter (n = 1 or 3); wall distance below one half: 7 x 7 (y, xi) sums
-    // of the opposite populations per node, exchanged through `sums` for the x filter (a sum of
-    // 7 x 7 x 7 terms per thread otherwise).
-    // Returns whether the row is set, with the populations (full values) in out.
+    // One flag type of the BFL rows (C/evolution.h:505-572) of a whole row y at plane z <= 1. dst / src:
+    // populations set and their opposites, the first without and the other two with an x filter (N3 = 1
+    // or 3). Returns whether the row is set, with the populations (full values) in out.
     template <int N3>
     __device__ __forceinline__ bool bfl_type(V2 *out, int fl, const int (&dst)[N3], const int (&src)[N3], const int (&xset)[N3],
-                                             int yset, int zset, int x0, int y, int z, int row, float *sums) const {
+                                             int yset, int zset, int x0, int y, int z) const {
         const int NY = k.NY, nb = 2*k.NYD6, r = z*k.NYD6 + y + 3;
         if (T.bfl_flag[fl*nb + r] != 1) return false;
         const size_t N = (size_t)NX*NY*k.NZ;
@@ -496,48 +535,11 @@ struct RoleKernel {
             for (int m = 0; m < N3; m++) out[m] = V2(c0)*ld2g<S>(nd + src[m]*N, src[m]) + V2(c1)*ld2g<S>(nd + dst[m]*N, dst[m]);
         }
         if (q < 0.5f) {
-            const int iy = k.bfl_mode ? r : y + 3;   // reference: X weights at [i], Y weights at [j]
-            V2 g[N3];
-#pragma unroll
-            for (int m = 0; m < N3; m++) g[m] = V2(0.f);
+            const int iy = k.bfl_mode ? r : y + 3;   // reference: Y weights at [j]
+            out[0] = bfl_y_xi(src[0], yset, zset, x0, y, r, iy);
+            if constexpr (N3 == 3)
 #pragma unroll 1
-            for (int c = 0; c < 7; c++) {
-                V2 in[N3];
-#pragma unroll
-                for (int m = 0; m < N3; m++) in[m] = V2(0.f);
-#pragma unroll
-                for (int b = 0; b < 7; b++) {
-                    int yy = y - 3 + b;
-                    yy = yy < 0 ? yy + NY : (yy >= NY ? yy - NY : yy);
-                    const V2 wv = V2(bw(yset, b, iy));
-                    const S *p = fo + ((size_t)c*NY + yy)*NX + x0;
-#pragma unroll
-                    for (int m = 0; m < N3; m++) in[m] = wv*ld2g<S>(p + src[m]*N, src[m]) + in[m];
-                }
-                const V2 wz = V2(bw(zset, c, r));
-#pragma unroll
-                for (int m = 0; m < N3; m++) g[m] = wz*in[m] + g[m];
-            }
-            out[0] = g[0];
-            if constexpr (N3 == 3) {
-                float *s = sums + row*NX;   // [2][512]: two populations
-                row_sync(row);              // the row's previous sums have been read
-                *(float2 *)(s + x0) = g[1].v;
-                *(float2 *)(s + 512 + x0) = g[2].v;
-                row_sync(row);
-#pragma unroll
-                for (int m = 1; m < 3; m++) {
-                    float o[2];
-#pragma unroll
-                    for (int l = 0; l < 2; l++) {
-                        const int ix = k.bfl_mode ? r : x0 + l + 3;
-                        o[l] = 0.f;
-#pragma unroll
-                        for (int a = 0; a < 7; a++) o[l] += bw(xset[m], a, ix)*s[(m - 1)*512 + ((x0 + l - 3 + a) & (NX - 1))];
-                    }
-                    out[m] = V2(o[0], o[1]);
-                }
-            }
+                for (int m = 1; m < 3; m++) out[m] = bfl_x_y_xi(m == 1 ? src[1] : src[2], m == 1 ? xset[1] : xset[2], yset, zset, x0, y, r, iy);
         }
         return q > 0.5f || q < 0.5f;
     }
@@ -551,7 +553,7 @@ struct RoleKernel {
         V2 bounce[5];      // 5, 11, 12, 15, 16 at z = 0
         unsigned set[2];   // BFL types set at plane z
     };
-    __device__ __forceinline__ void prepare_wall(Wall &w, int z0, int z1, int x0, int y, int row, float *sums) const {
+    __device__ __forceinline__ void prepare_wall(Wall &w, int z0, int z1, int x0, int y) const {
         const size_t N = (size_t)NX*k.NY*k.NZ;
         if (z0 == 0) {
             const S *b = fo + ((size_t)y*NX + x0);
@@ -564,10 +566,10 @@ struct RoleKernel {
 #pragma unroll 1
         for (int z = z0; z < z1; z++) {
             V2 *v = w.v[z];
-            unsigned m = bfl_type<3>(v, 0, {3, 7, 8}, {4, 10, 9}, {0, B_XB37, B_XB38}, B_YB378, B_XIB378, x0, y, z, row, sums) ? 1u : 0u;
-            m |= bfl_type<3>(v + 3, 1, {4, 9, 10}, {3, 8, 7}, {0, B_XB49, B_XB410}, B_YB4910, B_XIB4910, x0, y, z, row, sums) ? 2u : 0u;
-            m |= bfl_type<1>(v + 6, 2, {15}, {18}, {0}, B_YB15, B_XIB15, x0, y, z, row, sums) ? 4u : 0u;
-            m |= bfl_type<1>(v + 7, 3, {16}, {17}, {0}, B_YB16, B_XIB16, x0, y, z, row, sums) ? 8u : 0u;
+            unsigned m = bfl_type<3>(v, 0, {3, 7, 8}, {4, 10, 9}, {0, B_XB37, B_XB38}, B_YB378, B_XIB378, x0, y, z) ? 1u : 0u;
+            m |= bfl_type<3>(v + 3, 1, {4, 9, 10}, {3, 8, 7}, {0, B_XB49, B_XB410}, B_YB4910, B_XIB4910, x0, y, z) ? 2u : 0u;
+            m |= bfl_type<1>(v + 6, 2, {15}, {18}, {0}, B_YB15, B_XIB15, x0, y, z) ? 4u : 0u;
+            m |= bfl_type<1>(v + 7, 3, {16}, {17}, {0}, B_YB16, B_XIB16, x0, y, z) ? 8u : 0u;
             w.set[z] = m;
         }
     }
@@ -675,7 +677,7 @@ struct RoleKernel {
         L.own = L.row >= P.yskip;
         if (P.ta <= 1) {
             Wall wall;
-            if (L.own) prepare_wall(wall, P.ta, min(P.tb, 2), L.x0, L.y, L.row, (float *)(smem + LY::bfl_off));
+            if (L.own) prepare_wall(wall, P.ta, min(P.tb, 2), L.x0, L.y);
             collide_targets<true>(smem, P, P.ta, min(P.tb, 2), L, lane, sc, ub, mass, faulted, &wall);
         }
         collide_targets<false>(smem, P, max(P.ta, 2), P.tb, L, lane, sc, ub, mass, faulted, nullptr);

@@ -102,6 +102,7 @@ def load():
         "islbm_diagnostics": [vp, dp],
         "islbm_fault_drill": [vp, ip],
         "islbm_step_kernel": [vp, ctypes.POINTER(ip)],
+        "islbm_use_paired": [vp],
         "islbm_diagnostics_noalloc": [vp, dp],
         "islbm_write_tecplot_ascii": [vp, ctypes.c_char_p],
         "islbm_write_tecplot_plt": [vp, ctypes.c_char_p],

@@ -290,14 +290,16 @@ cudaError_t xfer_buffer(islbm_handle *h) {
 // Device address of a caller's pinned buffer of n doubles, else null. The conversion kernels store into
 // such a buffer directly: one pass instead of a conversion and a copy, and none of the copies of
 // 600 MB and more that ran at 4 to 45 instead of 180 GB/s every other time (fields of 384x384x512: 13
-// to 170 ms, by stores 12.6 ms each time).
+// to 170 ms, by stores 12.6 ms each time). A buffer that does not start at a double's boundary, or that the
+// device may not write, is left to the copy: a store there would fault.
 double *pinned_alias(double *out, size_t n) {
+    if ((uintptr_t)out % sizeof(double) != 0) return nullptr;
     cudaPointerAttributes a{};
     if (cudaPointerGetAttributes(&a, out) != cudaSuccess) {
         (void)cudaGetLastError();
         return nullptr;
     }
-    if (a.type != cudaMemoryTypeHost || !a.devicePointer) return nullptr;
+    if (a.type != cudaMemoryTypeHost || !a.devicePointer || (uintptr_t)a.devicePointer % sizeof(double) != 0) return nullptr;
     // the buffer has to lie in one pinned range: a copy also takes one that is pinned in part, or in pieces
     static const PFN_cuPointerGetAttribute_v4000 attribute = []() -> PFN_cuPointerGetAttribute_v4000 {
         void *fn = nullptr;
@@ -309,10 +311,13 @@ double *pinned_alias(double *out, size_t n) {
     }();
     CUdeviceptr start = 0;
     size_t size = 0;
+    unsigned long long access = 0;
     const CUdeviceptr at = (CUdeviceptr)a.devicePointer;
     if (!attribute || attribute(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at) != CUDA_SUCCESS ||
-        attribute(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at) != CUDA_SUCCESS)
+        attribute(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at) != CUDA_SUCCESS ||
+        attribute(&access, CU_POINTER_ATTRIBUTE_ACCESS_FLAGS, at) != CUDA_SUCCESS)
         return nullptr;
+    if ((access & CU_MEM_ACCESS_FLAGS_PROT_READWRITE) != CU_MEM_ACCESS_FLAGS_PROT_READWRITE) return nullptr;
     if (at < start || at - start > size || size - (at - start) < n*sizeof(double)) return nullptr;
     return (double *)a.devicePointer;
 }

@@ -547,7 +547,6 @@ namespace islbm {
 int handle_init(const islbm_params *p, islbm_handle *h) { return init_impl(p, h); }
 void handle_free(islbm_handle *h) { free_handle_impl(h); }
 int report_cuda(cudaError_t e, const char *what) { return cuda_fail(e, what); }
-cudaError_t handle_xfer(islbm_handle *h) { return xfer_buffer(h); }
 double *pinned_device_alias(double *out, size_t n) { return pinned_alias(out, n); }
 void unique_to_reference_layout(const islbm_handle *h, const double *u, double *r) { unique_to_reference(h, u, r); }
 void reference_to_unique_layout(const islbm_handle *h, const double *r, double *u) { reference_to_unique(h, r, u); }

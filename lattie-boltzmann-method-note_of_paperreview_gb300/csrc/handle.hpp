@@ -52,8 +52,6 @@ namespace islbm {
 // init/teardown used by the serving loop as well as islbm_init/islbm_destroy
 int handle_init(const islbm_params *p, islbm_handle *h);
 void handle_free(islbm_handle *h);
-// the handle's transfer buffer (h->xfer, N doubles), allocated on first use
-cudaError_t handle_xfer(islbm_handle *h);
 // device address of a caller's pinned buffer of n doubles, else null
 double *pinned_device_alias(double *out, size_t n);
 // record a CUDA failure for islbm_status_string and map it to a status

@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <cerrno>
 #include <cmath>
+#include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <string>
@@ -196,28 +197,26 @@ int islbm_stats_mean(islbm_handle *h, int quantity, double *out, int layout) {
     if (!h->stats || h->stats_samples == 0) return report_status(ISLBM_ERR_NOT_SUPPORTED, "no statistics samples");
     cudaError_t e = cudaSetDevice(h->device);
     if (e != cudaSuccess) return report_cuda(e, "cudaSetDevice");
-    // scaled on the device and copied straight into the caller's buffer (unique layout): the detour
-    // through a host vector took 0.70 ms per quantity of 128x64x96, four fifths of a window's read
+    // A pinned buffer is written by the device, scaled; into any other the sums are copied straight and scaled
+    // there, without device memory of its own (callers may have none left). A detour through a host vector
+    // took 0.70 ms per quantity of 128x64x96, four fifths of a window's read.
     const double inv = 1.0/(double)h->stats_samples;
-    std::vector<double> mean(layout == ISLBM_LAYOUT_REFERENCE ? h->N : 0);
-    double *dst = mean.empty() ? out : mean.data();
-    double *direct = mean.empty() ? pinned_device_alias(out, h->N) : nullptr;
-    e = direct ? cudaSuccess : handle_xfer(h);
-    if (e == cudaErrorMemoryAllocation) {   // no device memory for the buffer: scaled on the host
-        (void)cudaGetLastError();
-        e = cudaMemcpyAsync(dst, h->stats + (size_t)quantity*h->N, h->N*sizeof(double), cudaMemcpyDeviceToHost, h->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-        if (e == cudaSuccess)
-            for (size_t i = 0; i < h->N; i++) dst[i] *= inv;
-    } else if (e == cudaSuccess) {
-        const unsigned grid = (unsigned)std::min<size_t>(4096, (h->N + 255)/256);
-        mean_kernel<<<grid, 256, 0, h->stream>>>(h->stats + (size_t)quantity*h->N, direct ? direct : h->xfer, h->N, inv);
+    const double *sum = h->stats + (size_t)quantity*h->N;
+    if (double *direct = layout == ISLBM_LAYOUT_UNIQUE ? pinned_device_alias(out, h->N) : nullptr) {
+        mean_kernel<<<(unsigned)std::min<size_t>(4096, (h->N + 255)/256), 256, 0, h->stream>>>(sum, direct, h->N, inv);
         e = cudaGetLastError();
-        if (e == cudaSuccess && !direct) e = cudaMemcpyAsync(dst, h->xfer, h->N*sizeof(double), cudaMemcpyDeviceToHost, h->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+        return e == cudaSuccess ? ISLBM_OK : report_cuda(e, "statistics read");
     }
+    const bool in_place = layout == ISLBM_LAYOUT_UNIQUE && (uintptr_t)out % sizeof(double) == 0;
+    std::vector<double> mean(in_place ? 0 : h->N);
+    double *dst = in_place ? out : mean.data();
+    e = cudaMemcpyAsync(dst, sum, h->N*sizeof(double), cudaMemcpyDeviceToHost, h->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) return report_cuda(e, "statistics read");
+    for (size_t i = 0; i < h->N; i++) dst[i] *= inv;
     if (layout == ISLBM_LAYOUT_REFERENCE) unique_to_reference_layout(h, mean.data(), out);
+    else if (!in_place) std::memcpy(out, mean.data(), h->N*sizeof(double));
     return ISLBM_OK;
 }
 

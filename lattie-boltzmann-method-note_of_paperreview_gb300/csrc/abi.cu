@@ -300,7 +300,7 @@ double *pinned_alias(double *out, size_t n) {
         return nullptr;
     }
     if (a.type != cudaMemoryTypeHost || !a.devicePointer || (uintptr_t)a.devicePointer % sizeof(double) != 0) return nullptr;
-    // the buffer has to lie in one pinned range: a copy also takes one that is pinned in part, or in pieces
+    // the buffer has to lie in one pinned range; one that is pinned in part, or in pieces, is left to the copy
     static const PFN_cuPointerGetAttribute_v4000 attribute = []() -> PFN_cuPointerGetAttribute_v4000 {
         void *fn = nullptr;
         cudaDriverEntryPointQueryResult q;
@@ -386,8 +386,7 @@ int copy_macro(islbm_handle *h, int which, double *out, int layout) {
         return ISLBM_OK;
     }
     if (layout == ISLBM_LAYOUT_UNIQUE) {   // FP64 fields: as they are
-        CK(cudaMemcpyAsync(out, h->macros[which], N*8, cudaMemcpyDeviceToHost, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
+        CK(copy_out(h, (const double *)h->macros[which], out));
         return ISLBM_OK;
     }
     std::vector<double> tmp(N);
@@ -548,6 +547,19 @@ int handle_init(const islbm_params *p, islbm_handle *h) { return init_impl(p, h)
 void handle_free(islbm_handle *h) { free_handle_impl(h); }
 int report_cuda(cudaError_t e, const char *what) { return cuda_fail(e, what); }
 double *pinned_device_alias(double *out, size_t n) { return pinned_alias(out, n); }
+// N doubles from the device to a caller's buffer, finished on return. A buffer that is pinned in part or in several
+// pieces is refused by the copy ("invalid argument") and filled through a pageable one.
+cudaError_t copy_out(islbm_handle *h, const double *src, double *out) {
+    const size_t bytes = h->N*sizeof(double);
+    cudaError_t e = cudaMemcpyAsync(out, src, bytes, cudaMemcpyDeviceToHost, h->stream);
+    if (e != cudaErrorInvalidValue) return e == cudaSuccess ? cudaStreamSynchronize(h->stream) : e;
+    (void)cudaGetLastError();
+    std::vector<double> tmp(h->N);
+    e = cudaMemcpyAsync(tmp.data(), src, bytes, cudaMemcpyDeviceToHost, h->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    if (e == cudaSuccess) std::memcpy(out, tmp.data(), bytes);
+    return e;
+}
 void unique_to_reference_layout(const islbm_handle *h, const double *u, double *r) { unique_to_reference(h, u, r); }
 void reference_to_unique_layout(const islbm_handle *h, const double *r, double *u) { reference_to_unique(h, r, u); }
 int report_status(int status, const char *msg) {

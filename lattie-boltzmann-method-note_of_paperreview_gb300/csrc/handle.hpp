@@ -54,6 +54,8 @@ int handle_init(const islbm_params *p, islbm_handle *h);
 void handle_free(islbm_handle *h);
 // device address of a caller's pinned buffer of n doubles, else null
 double *pinned_device_alias(double *out, size_t n);
+// N doubles from the device to a caller's buffer, finished on return
+cudaError_t copy_out(islbm_handle *h, const double *src, double *out);
 // record a CUDA failure for islbm_status_string and map it to a status
 int report_cuda(cudaError_t e, const char *what);
 // record a message for islbm_status_string and return `status`

@@ -211,8 +211,7 @@ int islbm_stats_mean(islbm_handle *h, int quantity, double *out, int layout) {
     const bool in_place = layout == ISLBM_LAYOUT_UNIQUE && (uintptr_t)out % sizeof(double) == 0;
     std::vector<double> mean(in_place ? 0 : h->N);
     double *dst = in_place ? out : mean.data();
-    e = cudaMemcpyAsync(dst, sum, h->N*sizeof(double), cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    e = copy_out(h, sum, dst);
     if (e != cudaSuccess) return report_cuda(e, "statistics read");
     for (size_t i = 0; i < h->N; i++) dst[i] *= inv;
     if (layout == ISLBM_LAYOUT_REFERENCE) unique_to_reference_layout(h, mean.data(), out);

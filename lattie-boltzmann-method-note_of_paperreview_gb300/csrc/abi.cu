@@ -624,7 +624,7 @@ int islbm_step(islbm_handle *h, int nsteps) {
         L.fn = h->fbuf[1 - h->cur];
         L.pmaps = h->roles ? h->rmaps.for_buffer(L.fo) : h->paired ? h->pmaps.for_buffer(L.fo) : nullptr;
         L.n = n;
-        L.launch = ++h->launches;
+        L.seat_set = h->seat_set ^= 1u;
         L.mass = h->p.mass_interval > 0 && (n % (unsigned long long)h->p.mass_interval) == 0ULL;
         L.macros_on = (s == nsteps - 1);
         for (int m = 0; m < 4; m++) L.macros[m] = h->macros[m];

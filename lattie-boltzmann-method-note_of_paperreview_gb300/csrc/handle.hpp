@@ -29,7 +29,7 @@ struct islbm_handle {
     StepConst k{};
     int cur = 0;
     unsigned long long steps = 0;
-    unsigned long long launches = 0;   // step launches so far (seats of step_roles.cuh)
+    unsigned seat_set = 0;     // seats of the last step launch (step_roles.cuh)
     bool use_tiled = false;    // a tiled kernel (shared-memory tiles, TMEM ring) steps this solve
     bool paired = false;       // ... the paired-node one (step_pair.cu), else step_tiled.cu
     double *stats = nullptr;   // time-average accumulators, ISLBM_STAT_COUNT x N (allocated on first use)

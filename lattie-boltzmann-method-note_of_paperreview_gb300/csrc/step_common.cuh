@@ -82,13 +82,13 @@ struct Ctrl {
     unsigned int fault;      // set when a pipeline wait gave up (bounded waits)
 };
 
-// Behind the controller in its allocation: the seats of a step launch whose blocks choose their work by
-// the SM they run on (step_roles.cuh; the number of the last launch that took each), and the partial
-// sums (plane sum, mass) of a step's blocks or work items.
+// Behind the controller in its allocation: two sets of seats for step launches whose blocks choose their work by
+// the SM they run on (step_roles.cuh; 1: taken by a block of the launch that uses the set), and the
+// partial sums (plane sum, mass) of a step's blocks or work items.
 constexpr int MAX_SEATS = 256, MAX_PARTS = 2048;
-constexpr size_t SEATS_OFF = (sizeof(Ctrl) + 255)/256*256, PARTS_OFF = SEATS_OFF + MAX_SEATS*sizeof(unsigned long long);
+constexpr size_t SEATS_OFF = (sizeof(Ctrl) + 255)/256*256, PARTS_OFF = SEATS_OFF + 2*MAX_SEATS*sizeof(unsigned);
 constexpr size_t CTRL_BYTES = PARTS_OFF + MAX_PARTS*sizeof(double2);
-__device__ __forceinline__ unsigned long long *ctrl_seats(Ctrl *c) { return (unsigned long long *)((char *)c + SEATS_OFF); }
+__device__ __forceinline__ unsigned *ctrl_seats(Ctrl *c, unsigned set) { return (unsigned *)((char *)c + SEATS_OFF) + set*MAX_SEATS; }
 __device__ __forceinline__ double2 *ctrl_parts(Ctrl *c) { return (double2 *)((char *)c + PARTS_OFF); }
 
 template <class C> struct Tables {
@@ -318,9 +318,10 @@ __device__ __forceinline__ void end_of_step(Ctrl *ctrl, const StepConst &k, unsi
 // The same in a fixed order, so that the controller's sums (and every result) do not depend on which
 // block comes first: block or work item `index` of `total` stores its partial sums, the last one to
 // finish adds them by index. Run by a group of NTHREADS threads (a multiple of 32, tid = 0 ..
-// NTHREADS - 1) synchronised by `sync`. More parts than MAX_PARTS are added atomically.
+// NTHREADS - 1) synchronised by `sync`. More parts than MAX_PARTS are added atomically. Returns whether
+// this block or item was the last.
 template <int NTHREADS, class SYNC>
-__device__ __forceinline__ void end_of_step_ordered(Ctrl *ctrl, const StepConst &k, unsigned long long n, double ub, double mass,
+__device__ __forceinline__ bool end_of_step_ordered(Ctrl *ctrl, const StepConst &k, unsigned long long n, double ub, double mass,
                                                     bool mass_step, unsigned index, unsigned total, int tid, SYNC &&sync) {
     __shared__ double gred[2][NTHREADS/32];
     __shared__ bool glast;
@@ -343,7 +344,7 @@ __device__ __forceinline__ void end_of_step_ordered(Ctrl *ctrl, const StepConst 
         glast = atomicAdd(&ctrl->done, 1u) == total - 1u;
     }
     sync();
-    if (!glast) return;
+    if (!glast) return false;
     __threadfence();
     double s = 0.0, m = 0.0;
     if (ordered) {
@@ -361,6 +362,7 @@ __device__ __forceinline__ void end_of_step_ordered(Ctrl *ctrl, const StepConst 
         if (ordered) ctrl->ub_slot[n & 1ULL] = s;
         finish_step(ctrl, k, n, mass_step, m);
     }
+    return true;
 }
 
 }  // namespace islbm

@@ -16,7 +16,7 @@ struct StepLaunch {
     StepConst k;
     Ctrl *ctrl;                // device
     unsigned long long n;      // 1-based number of the step being computed
-    unsigned long long launch; // number of this step launch of the handle (1, 2, ...)
+    unsigned seat_set;         // 0, 1, 0, ... over the step launches of the handle
     bool les, macros_on, mass;
     void *macros[4];           // rho, u, v, w (compute type) when macros_on
     const void *tiled;         // TiledConst for the tiled kernel

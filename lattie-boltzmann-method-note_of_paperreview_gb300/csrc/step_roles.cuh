@@ -137,7 +137,7 @@ struct RoleKernel {
     Ctrl *ctrl;
     float *rho_out, *u_out, *v_out, *w_out;
     int macros_on, mass_on;
-    unsigned long long launch;   // number of this launch of the solve
+    unsigned seat_set;         // seats of this launch
 
     // position in a ring of N stages: index and phase parity
     template <int N> struct Stage {
@@ -717,8 +717,11 @@ struct RoleKernel {
     // the halo rows they read at the same time (256x128x192, without dependent launches: FP32 181
     // -> 178, FP16 181 -> 171 us per step; with an arbitrary placement 230 and 275, and dependent
     // launches place CTAs as SMs become free). Any placement is valid: a CTA takes the seat of its
-    // SM or the next free one; a seat is free to a launch that no earlier or equal number holds.
-    // (Grids smaller than the GPU go by block number.) The claim runs beside the CTA's set-up.
+    // SM or the next free one. (Grids smaller than the GPU go by block number.) The claim runs beside the
+    // CTA's set-up. Launches take the two sets of seats in turn; the last CTA of a launch empties its set,
+    // before the launch after next, which takes that set again, can start (a launch starts once every CTA of
+    // the one before is past its wait for the end of the one before that). So nothing in a launch's
+    // arguments marks a seat as taken, and a captured pair of launches can be replayed.
     __device__ __forceinline__ void claim_seat(unsigned char *smem, int tid) const {
         if (tid != 32) return;   // not the warp that allocates tensor memory
         const unsigned n = gridDim.x;
@@ -726,9 +729,9 @@ struct RoleKernel {
         if (tc.seats && n <= (unsigned)MAX_SEATS) {
             unsigned sm;
             asm volatile("mov.u32 %0, %smid;" : "=r"(sm));
-            unsigned long long *seats = ctrl_seats(ctrl);
+            unsigned *seats = ctrl_seats(ctrl, seat_set);
             s = sm < n ? sm : n - 1;
-            for (unsigned i = 1; i < n && atomicMax(seats + s, launch) >= launch; i++) s = s + 1 == n ? 0 : s + 1;
+            for (unsigned i = 1; i < n && atomicExch(seats + s, 1u) != 0u; i++) s = s + 1 == n ? 0 : s + 1;
         }
         *(volatile int *)(smem + LY::flag_off + 4) = (int)s;
     }
@@ -778,8 +781,9 @@ struct RoleKernel {
             // these became free, which scatters neighbouring tiles
             grid_dependency_trigger();
             ring_free(smem, tid);
-            end_of_step_ordered<COLLIDE_THREADS>(ctrl, k, tc.n, ub_total, mass_total, mass_on != 0, (unsigned)seat, gridDim.x, tid,
-                                                 [] { bar_sync(BAR_COLLIDE, COLLIDE_THREADS); });
+            const bool last = end_of_step_ordered<COLLIDE_THREADS>(ctrl, k, tc.n, ub_total, mass_total, mass_on != 0, (unsigned)seat,
+                                                                   gridDim.x, tid, [] { bar_sync(BAR_COLLIDE, COLLIDE_THREADS); });
+            if (last && tid < MAX_SEATS) ctrl_seats(ctrl, seat_set)[tid] = 0u;   // (every CTA took its seat long ago)
         } else if (warp < FRONT_WARP) {
             if (warp < FILTER_WARP0 + 4) regs_dec<Regs<S>::rows>();
             else regs_dec<Regs<S>::quads>();
@@ -933,7 +937,7 @@ struct RoleOps {
         K.rho_out = (float *)L.macros[0]; K.u_out = (float *)L.macros[1];
         K.v_out = (float *)L.macros[2]; K.w_out = (float *)L.macros[3];
         K.macros_on = L.macros_on; K.mass_on = L.mass;
-        K.launch = L.launch;
+        K.seat_set = L.seat_set;
         RoleTM T;
         std::memset((void *)&T, 0, sizeof(T));
         if (L.pmaps) std::memcpy((void *)T.m, L.pmaps, sizeof(T.m));

@@ -24,6 +24,7 @@ def test_chains_of_steps_match_single_steps(islbm_lib, prec, nx, ny, nz, les):
         b.step(60)
         b.sync()
         fa, fb = a.populations(), b.populations()
+        assert np.isfinite(fa).all()
         np.testing.assert_array_equal(fa, fb)
         for _ in range(5):
             b.step(200)

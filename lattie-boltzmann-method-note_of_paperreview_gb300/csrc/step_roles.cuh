@@ -82,7 +82,7 @@ __host__ __device__ constexpr int FQ(int i) {
 //   NFS front stages; NTS target stages (populations 0, 1, 2 as TY rows, then the rows' duplicated
 //   xi weights, TY x 128 floats); ybuf [2][TY][2][NX/2] float4: streamwise-filtered (7, 8, 9, 10)
 //   by plane parity, the even and the odd node of each pair apart (consecutive threads, consecutive
-//   16 bytes); mbarriers; timeout flag and TMEM address.
+//   16 bytes); a double2 of sums per collide thread; mbarriers; timeout flag and TMEM address.
 template <class S, int NXC>
 struct RLay {
     static constexpr int NX = NXC, PR = NX/2, TY = 512/NX;
@@ -96,18 +96,19 @@ struct RLay {
     static constexpr int w_off = up128(3*plain_pop);
     static constexpr int target_bytes = w_off + TY*512;
     static constexpr unsigned target_tx = (unsigned)(3*plain_pop + TY*512);
-    static constexpr int ybuf_bytes = 2*512*16;
+    static constexpr int ybuf_bytes = 2*512*16, sums_bytes = COLLIDE_THREADS*16;
     // front stages: as many as fit, up to three. The copies of a plane take about 2.5 us from issue to
     // completion under load, longer than a plane's work: with two stages the copies' latency set
     // the pace (FP32 256x128x192 without collisions and stores 184 us per step, with them 207)
-    static constexpr int room = 227*1024 - ybuf_bytes - 1536;
+    static constexpr int room = 227*1024 - ybuf_bytes - sums_bytes - 1536;
     static constexpr int fit = (room - 2*target_bytes)/front_bytes;
     static constexpr int NFS = fit > 3 ? 3 : fit;
     static constexpr int NTS = NFS*front_bytes + 4*target_bytes <= room ? 4 : 2;
     static_assert(NFS >= 2, "two front stages");
     static constexpr int target_off = NFS*front_bytes;
     static constexpr int ybuf_off = target_off + NTS*target_bytes;
-    static constexpr int bar_off = ybuf_off + ybuf_bytes;
+    static constexpr int sums_off = ybuf_off + ybuf_bytes;
+    static constexpr int bar_off = sums_off + sums_bytes;
     // mbarriers: front full, front empty, target full, target empty, ring full and ring free per
     // lane quarter and slot
     static constexpr int B_FF = 0, B_FE = NFS, B_TF = 2*NFS, B_TE = B_TF + NTS, B_RF = B_TE + NTS, B_RE = B_RF + 4*SLOTS;
@@ -610,7 +611,7 @@ struct RoleKernel {
             *(float2 *)((char *)rho_out + moff) = rho.v; *(float2 *)((char *)u_out + moff) = u1.v;
             *(float2 *)((char *)v_out + moff) = v1.v; *(float2 *)((char *)w_out + moff) = w1.v;
         }
-        // column partials in FP32 (at most NZ terms), folded into FP64 once per piece
+        // column partials in FP32, at most FOLD terms (collide_piece)
         if (y == k.yplane) ub += (v1.v.x*T.dxf[x0] + v1.v.y*T.dxf[x0 + 1])*T.dzf[z];
         mass = mass + rho;   // a non-finite density makes the mass sum non-finite (checked once per piece)
     }
@@ -661,9 +662,24 @@ struct RoleKernel {
     }
     // All targets of a piece for collide warp `warp` (lane quarter warp % 4, row of the pair warp / 4);
     // seq0: ring sequence number of plane p0, tcount: target stages used before this piece. The wall
-    // planes run in a loop of their own, so that the main one carries none of their state.
+    // planes run in a loop of their own, so that the main one carries none of their state. The sums of the plane
+    // velocity and the density are added in FP32 over at most FOLD targets (the paired kernel's segments
+    // have 16 or more), then in FP64 in the thread's word `sums` in shared memory: a segment may be the
+    // whole column, 84 targets on 128x256x192. (In registers the FP64 sums cost 204 instead of 196 us there;
+    // FP32 sums with their rounding errors beside them 206 to 226.)
+    static constexpr int FOLD = 16;
     __device__ __forceinline__ void collide_piece(unsigned char *smem, const Piece &P, unsigned seq0, unsigned tcount, int warp, int lane,
-                                                  uint32_t tl, const Scal &sc, float &ub, V2 &mass, bool &faulted) const {
+                                                  uint32_t tl, const Scal &sc, double2 *sums, bool &faulted) const {
+        float ub = 0.f;
+        V2 mass = V2(0.f);
+        auto fold = [&] {
+            double2 s = *sums;
+            s.x += (double)ub;
+            s.y += (double)(mass.v.x + mass.v.y);
+            *sums = s;
+            ub = 0.f;
+            mass = V2(0.f);
+        };
         Pair L;
         L.w = warp & 3;
         L.i = 32*L.w + lane;
@@ -680,7 +696,13 @@ struct RoleKernel {
             if (L.own) prepare_wall(wall, P.ta, min(P.tb, 2), L.x0, L.y);
             collide_targets<true>(smem, P, P.ta, min(P.tb, 2), L, lane, sc, ub, mass, faulted, &wall);
         }
-        collide_targets<false>(smem, P, max(P.ta, 2), P.tb, L, lane, sc, ub, mass, faulted, nullptr);
+#pragma unroll 1
+        for (int t = max(P.ta, 2); t < P.tb; t += FOLD) {
+            collide_targets<false>(smem, P, t, min(t + FOLD, P.tb), L, lane, sc, ub, mass, faulted, nullptr);
+            fold();
+        }
+        if (P.tb <= 2) fold();   // a segment of wall planes only
+        if (!isfinite(sums->y)) ctrl->nonfinite = 1u;
     }
 
     // ---- CTA set-up and end ----
@@ -763,25 +785,20 @@ struct RoleKernel {
         if (warp < COLLIDE_WARPS) {
             regs_inc<Regs<S>::collide>();
             const uint32_t tl = tmem_base(smem) + ((uint32_t)(32*(warp & 3)) << 16) + 256u*(uint32_t)(warp >> 2);
-            double ub_total = 0.0, mass_total = 0.0;
+            double2 *sums = (double2 *)(smem + LY::sums_off) + tid;
+            *sums = make_double2(0.0, 0.0);
             const Scal sc = scalars();
             unsigned seq = 0, tcount = 0;
             for_items(seat, [&](const Piece &P) {
-                float ub = 0.f;
-                V2 mass = V2(0.f);
-                collide_piece(smem, P, seq, tcount, warp, lane, tl, sc, ub, mass, faulted);
+                collide_piece(smem, P, seq, tcount, warp, lane, tl, sc, sums, faulted);
                 seq += (unsigned)(P.p1 - P.p0 + 1);
                 tcount += (unsigned)(P.tb - P.ta);
-                const float m = mass.v.x + mass.v.y;
-                if (!isfinite(m)) ctrl->nonfinite = 1u;
-                ub_total += (double)ub;
-                mass_total += (double)m;
             });
             // the next step's CTAs may come now: triggered at the start, they took SMs one by one as
             // these became free, which scatters neighbouring tiles
             grid_dependency_trigger();
             ring_free(smem, tid);
-            const bool last = end_of_step_ordered<COLLIDE_THREADS>(ctrl, k, tc.n, ub_total, mass_total, mass_on != 0, (unsigned)seat,
+            const bool last = end_of_step_ordered<COLLIDE_THREADS>(ctrl, k, tc.n, sums->x, sums->y, mass_on != 0, (unsigned)seat,
                                                                    gridDim.x, tid, [] { bar_sync(BAR_COLLIDE, COLLIDE_THREADS); });
             if (last && tid < MAX_SEATS) ctrl_seats(ctrl, seat_set)[tid] = 0u;   // (every CTA took its seat long ago)
         } else if (warp < FRONT_WARP) {
@@ -870,17 +887,15 @@ step_roles_batch_kernel(const RoleBatchDesc<S, LES, NXC> *__restrict__ descs, co
         regs_inc<Regs<S>::collide>();
         const uint32_t tl = KT::tmem_base(smem) + ((uint32_t)(32*(warp & 3)) << 16) + 256u*(uint32_t)(warp >> 2);
         unsigned seq = 0, tcount = 0;
+        double2 *sums = (double2 *)(smem + KT::LY::sums_off) + tid;
         for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
             const typename KT::Piece P = load_item(it, w, tm);
             const auto sc = K.scalars();
-            float ub = 0.f;
-            V2 mass = V2(0.f);
-            K.collide_piece(smem, P, seq, tcount, warp, lane, tl, sc, ub, mass, faulted);
+            *sums = make_double2(0.0, 0.0);
+            K.collide_piece(smem, P, seq, tcount, warp, lane, tl, sc, sums, faulted);
             seq += (unsigned)(P.p1 - P.p0 + 1);
             tcount += (unsigned)(P.tb - P.ta);
-            const float m = mass.v.x + mass.v.y;
-            if (!isfinite(m)) K.ctrl->nonfinite = 1u;
-            end_of_step_ordered<COLLIDE_THREADS>(K.ctrl, K.k, K.tc.n, (double)ub, (double)m, K.mass_on != 0, (unsigned)w.y,
+            end_of_step_ordered<COLLIDE_THREADS>(K.ctrl, K.k, K.tc.n, sums->x, sums->y, K.mass_on != 0, (unsigned)w.y,
                                                  (unsigned)(descs[w.x].ntiles*descs[w.x].nseg), tid,
                                                  [] { bar_sync(BAR_COLLIDE, COLLIDE_THREADS); });
         }

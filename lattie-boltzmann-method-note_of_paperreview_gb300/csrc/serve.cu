@@ -13,7 +13,8 @@
 //      for the queue. A chunk ends at the next check or cap of any active solve, so every
 //      check of every solve spans exactly steps_per_chunk of its steps, whenever it arrived.
 // The launch shape of each batch (persistent CTAs per SM) is picked by a small autotuner that
-// times the candidates on the first steps of a new batch composition and caches the winner.
+// times the candidates on the first steps of a new batch composition and caches the winner (batches of the
+// role-specialised kernel: one CTA per SM).
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -336,8 +337,11 @@ cudaError_t launch_batch(Group *g, int grid, int macros_on) {
 // at most `budget` of them, their number returned in `launched`.
 int tune(islbm_server *s, Group *g, int budget, int &launched) {
     launched = 0;
+    // the role-specialised kernel fits one CTA per SM: more CTAs only repeat its set-up and ring fill (12 solves of
+    // 64x32x48 183.6 ms, 3 50.8; with 2 or 4 CTAs per SM 183.5 and 50.9; timing the candidates first 185.4 and 53.5)
+    if (g->roles) { g->grid = std::min(g->nitems, s->sms); return ISLBM_OK; }
     const std::string sig = std::to_string(g->precision) + "/" + std::to_string(g->NX) + "/" + std::to_string(g->les) +
-                            "/" + std::to_string(g->nitems);
+                            "/" + std::to_string(g->paired ? 1 : 0) + "/" + std::to_string(g->nitems);
     auto it = s->tuned_grid.find(sig);
     if (it != s->tuned_grid.end()) { g->grid = it->second; return ISLBM_OK; }
     const int cand[3] = {std::min(g->nitems, s->sms), std::min(g->nitems, 2*s->sms), std::min(g->nitems, 4*s->sms)};

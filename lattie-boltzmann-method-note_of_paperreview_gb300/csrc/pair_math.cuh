@@ -6,7 +6,7 @@
 
 #include <cuda_runtime.h>
 
-#include "collide.cuh"
+#include "mrt_d3q19.cuh"
 
 namespace islbm {
 
@@ -51,16 +51,12 @@ __device__ __forceinline__ V2 &operator-=(V2 &a, V2 b) { a = vsub(a, b); return 
 __device__ __forceinline__ V2 &operator+=(V2 &a, V2M m) { a = vfma(m.a, m.b, a); return a; }
 __device__ __forceinline__ V2 &operator-=(V2 &a, V2M m) { a = vfma(vneg(m.a), m.b, a); return a; }
 
-// per-lane reciprocal and square root (no packed forms)
-__device__ __forceinline__ V2 c_rcp(V2 a) { return V2(c_rcp(a.v.x), c_rcp(a.v.y)); }
-__device__ __forceinline__ V2 c_sqrt(V2 a) { return V2(c_sqrt(a.v.x), c_sqrt(a.v.y)); }
-
 // per-lane reciprocal and square root (no packed forms): the hardware approximations of the
 // scalar FP32 collision
 __device__ __forceinline__ V2 vrcp(V2 a) { return V2(__fdividef(1.f, a.v.x), __fdividef(1.f, a.v.y)); }
 __device__ __forceinline__ float sqrt_nn(float v) { return v > 0.f ? v*rsqrtf(v) : 0.f; }
 
-// Collision tail of C/evolution.h:597-652 for a node pair, the operator of collide_pairs
+// Collision tail of C/evolution.h:597-652 for a node pair, the operator of collide_node_pairs
 // (step_common.cuh) on packed pairs: mass correction, density and velocity from the opposite-
 // direction pair sums and differences, their non-equilibrium parts, the Smagorinsky rate from
 // Q = Pi:Pi (LES), the generated sparse MRT relaxation and the body force.

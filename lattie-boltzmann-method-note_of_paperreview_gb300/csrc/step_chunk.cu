@@ -433,7 +433,7 @@ struct Chunk {
         if (t <= 1) bfl_apply(F, L, t, bf);
         C rho, u1, v1, w1;
         if constexpr (sizeof(C) == 4) collide_node<C, LES>(F, rho_mod, f6, f12, (C)k.tau, (C)k.les_C, rho, u1, v1, w1);
-        else collide<LES>(F, rho_mod, f6, f12, (C)k.tau, (C)k.les_C, rho, u1, v1, w1);
+        else collide<LES>(F, rho_mod, f6, f12, k.tau, k.les_C, rho, u1, v1, w1);
 #pragma unroll
         for (int q = 0; q < 19; q++) store_f<S>((S *)((char *)fnq[q] + nd), 0, q, F[q]);
         if (macros_on) { rho_out[node] = rho; u_out[node] = u1; v_out[node] = v1; w_out[node] = w1; }

@@ -27,7 +27,7 @@
 //     reads a 7-plane ring of filtered node pairs kept in tensor memory (TMEM, 256 columns per
 //     128 threads: 7 planes x 16 directions x 2 nodes, plus the F1/F2 delay line) with the xi
 //     weights stored as duplicated pairs;
-//   * the collision of the pair runs in packed FP32x2 arithmetic (collide.cuh), results are
+//   * the collision of the pair runs in packed FP32x2 arithmetic (collide_x2), results are
 //     stored as node pairs (8-byte stores for FP32, 4-byte for FP16/BF16);
 //   * persistent CTAs, two per SM (one at NX = 384; TMEM bound), work items (wall-normal segment, tile) taken
 //     segment-major so that CTAs running together share their halo rows through L2.

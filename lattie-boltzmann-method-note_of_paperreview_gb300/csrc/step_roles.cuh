@@ -858,7 +858,7 @@ step_roles_batch_kernel(const RoleBatchDesc<S, LES, NXC> *__restrict__ descs, co
     KT::init(smem, tid);
     grid_dependency_wait();
     bool faulted = false;
-    // the descriptor of item `it` into K, by the 14 active warps together
+    // the descriptor of item `it` into K, by the 18 active warps together
     auto load_item = [&](int it, int2 &w, const CUtensorMap *&tm) {
         w = items[it];
         bar_sync(BAR_ITEM, ACTIVE_THREADS);   // every role is done with the previous item

@@ -25,7 +25,6 @@
 #include <cstring>
 #include <type_traits>
 
-#include "collide.cuh"
 #include "step_common.cuh"
 #include "step_launch.hpp"
 #include "step_tiled.hpp"
@@ -227,7 +226,7 @@ struct TiledKernel {
 #pragma unroll
         for (int q = 0; q < 19; q++) Fl[q] = F[q];
         float rho_s, u1, v1, w1;
-        collide_pairs<float, LES>(Fl, sc.rho_mod, sc.f6, sc.f12, sc.tau, sc.lesC, rho_s, u1, v1, w1);
+        collide_node_pairs<LES>(Fl, sc.rho_mod, sc.f6, sc.f12, sc.tau, sc.lesC, rho_s, u1, v1, w1);
 #pragma unroll
         for (int q = 0; q < 19; q++) store_f<S>(fnq[q], (unsigned)node, q, Fl[q]);
         if (macros_on) { rho_out[node] = rho_s; u_out[node] = u1; v_out[node] = v1; w_out[node] = w1; }

@@ -4,6 +4,7 @@ one-node-per-thread tiled kernel or of the gather kernel, bit for bit."""
 import numpy as np
 import pytest
 
+from conftest import rel_l2
 from test_chunk import params
 from test_chunk_order import CHUNK, GATHER, PAIRED, ROLES, TILED, run, step_kernel
 
@@ -21,6 +22,18 @@ def test_choice(islbm_lib, nx, ny, nz, fp32, half):
     for prec, want in (("fp32", fp32), ("fp16", half), ("bf16", half), ("fp64", CHUNK)):
         with islbm_lib.Solver(islbm_lib.default_params(**params(nx, ny, nz, precision=prec))) as s:
             assert step_kernel(islbm_lib, s) == want, prec
+
+
+@pytest.mark.parametrize("prec,tol", [("fp32", 2e-6), ("fp16", 2e-3)])
+@pytest.mark.parametrize("nx,ny,nz", [(32, 16, 16), (64, 12, 32), (128, 8, 56), (384, 8, 160)])
+def test_paired_grids_match_gather(islbm_lib, prec, tol, nx, ny, nz):
+    """The grids that the paired kernel still steps, with the tolerances of the formats."""
+    kw = params(nx, ny, nz, precision=prec, init_mode=1, seed=4, les_cs=0.1)
+    a = run(islbm_lib, GATHER, [20], kernel=islbm_lib.KERNEL_GATHER, **kw)
+    b = run(islbm_lib, PAIRED, [20], **kw)
+    assert np.isfinite(a[0]).all()
+    assert rel_l2(b[1][0], a[1][0]) <= tol
+    assert rel_l2(b[1][1:], a[1][1:]) <= 50*tol
 
 
 @pytest.mark.parametrize("prec", ["fp32", "fp16"])

@@ -142,7 +142,7 @@ struct Chunk {
     struct Col {
         int x, y, xl, yl;
         bool on, row;        // a column of the tile; phase A of FP32: a column of the grid
-        unsigned ro, xo[7];  // byte offsets within a plane: the row and, in a row, the spanwise stencil's nodes
+        unsigned ro, xo[7];  // byte offsets within a plane: the spanwise stencil's nodes (FP32: in a row, and the row's)
         unsigned yo[7];      // and the streamwise stencil's
     };
     // phase A, FP32: x filter of 7, 8, 9, 10 on planes p0 .. p0 + np - 1, rows y0 - 3 .. y0 + H + 2
@@ -461,11 +461,12 @@ struct Chunk {
             L.x = x0 + L.xl; L.y = y0 + L.yl;
             L.on = L.yl < cc.H && L.x < NX && L.y < NY;
             L.row = L.yl < P/cc.W && L.x < NX;
-            L.ro = (unsigned)(L.y*NX)*EB;
+            const unsigned row = (unsigned)(L.y*NX)*EB;
+            L.ro = GATHER ? row : 0u;
             if (GATHER ? L.row : L.on) {
 #pragma unroll
                 for (int a = 0; a < 7; a++) {
-                    L.xo[a] = (unsigned)wrap_any(L.x - 3 + a, NX)*EB;
+                    L.xo[a] = (unsigned)wrap_any(L.x - 3 + a, NX)*EB + (GATHER ? 0u : row);
                     L.yo[a] = (unsigned)(wrap_near(L.y - 3 + a, NY)*NX + L.x)*EB;
                 }
             }
@@ -473,8 +474,8 @@ struct Chunk {
             for (int t0 = ta; t0 < tb; t0 += CHUNK) {
                 const int t1 = min(t0 + CHUNK, tb);
                 const int pend = base(t1 - 1) + 7;
-                while (true) {
-                    const int pb = min(np + batch<C>(), pend);
+                // planes np .. pb - 1: quads, then ring values
+                auto planes = [&](int pb) {
                     if constexpr (GATHER) halo_rows(qb, np, pb - np, y0, L, g);
                     else halo_quads(qb, np, pb - np, x0, y0);
                     __syncthreads();   // quads complete; every thread is done with the previous chunk's targets
@@ -483,9 +484,13 @@ struct Chunk {
                             filter(L, qb + (GATHER ? ((p - np)*(cc.H + 6) + L.yl)*cc.W : ((p - np)*cc.H + L.yl)*(cc.W + 6)) + L.xl, p,
                                    ring + (size_t)(p % RING)*4*P + c);
                     np = pb;
-                    if (np >= pend) break;
-                    __syncthreads();   // quads free
-                }
+                };
+                if constexpr (GATHER)
+                    while (pend - np > batch<C>()) {
+                        planes(np + batch<C>());
+                        __syncthreads();   // quads free
+                    }
+                planes(pend);
                 if constexpr (GATHER) { if (L.on) y_of_xi(L, t0, t1, g, f34 + c); }
                 __syncthreads();   // ring complete, quads free
                 if (t0 <= 1) {

@@ -611,7 +611,7 @@ struct RoleKernel {
             *(float2 *)((char *)rho_out + moff) = rho.v; *(float2 *)((char *)u_out + moff) = u1.v;
             *(float2 *)((char *)v_out + moff) = v1.v; *(float2 *)((char *)w_out + moff) = w1.v;
         }
-        // column partials in FP32, at most FOLD terms (collide_piece)
+        // column partials in FP32, at most 16 terms (collide_piece)
         if (y == k.yplane) ub += (v1.v.x*T.dxf[x0] + v1.v.y*T.dxf[x0 + 1])*T.dzf[z];
         mass = mass + rho;   // a non-finite density makes the mass sum non-finite (checked once per piece)
     }
@@ -663,11 +663,11 @@ struct RoleKernel {
     // All targets of a piece for collide warp `warp` (lane quarter warp % 4, row of the pair warp / 4);
     // seq0: ring sequence number of plane p0, tcount: target stages used before this piece. The wall
     // planes run in a loop of their own, so that the main one carries none of their state. The sums of the plane
-    // velocity and the density are added in FP32 over at most FOLD targets (the paired kernel's segments
-    // have 16 or more), then in FP64 in the thread's word `sums` in shared memory: a segment may be the
+    // velocity and the density are added in FP32 over FOLD targets, 16 with the two wall planes (the paired
+    // kernel's segments have 16 or more), then in FP64 in the thread's word `sums` in shared memory: a segment may be the
     // whole column, 84 targets on 128x256x192. (In registers the FP64 sums cost 204 instead of 196 us there;
     // FP32 sums with their rounding errors beside them 206 to 226.)
-    static constexpr int FOLD = 16;
+    static constexpr int FOLD = 14;
     __device__ __forceinline__ void collide_piece(unsigned char *smem, const Piece &P, unsigned seq0, unsigned tcount, int warp, int lane,
                                                   uint32_t tl, const Scal &sc, double2 *sums, bool &faulted) const {
         float ub = 0.f;

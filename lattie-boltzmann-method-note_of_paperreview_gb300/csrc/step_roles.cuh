@@ -82,7 +82,8 @@ __host__ __device__ constexpr int FQ(int i) {
 //   NFS front stages; NTS target stages (populations 0, 1, 2 as TY rows, then the rows' duplicated
 //   xi weights, TY x 128 floats); ybuf [2][TY][2][NX/2] float4: streamwise-filtered (7, 8, 9, 10)
 //   by plane parity, the even and the odd node of each pair apart (consecutive threads, consecutive
-//   16 bytes); a double2 of sums per collide thread; mbarriers; timeout flag and TMEM address.
+//   16 bytes); a double2 of sums per collide thread; near wall rows: one sum per collide
+//   thread, their weights, lists of two planes; mbarriers; timeout flag and TMEM address.
 template <class S, int NXC>
 struct RLay {
     static constexpr int NX = NXC, PR = NX/2, TY = 512/NX;
@@ -97,10 +98,11 @@ struct RLay {
     static constexpr int target_bytes = w_off + TY*512;
     static constexpr unsigned target_tx = (unsigned)(3*plain_pop + TY*512);
     static constexpr int ybuf_bytes = 2*512*16, sums_bytes = COLLIDE_THREADS*16;
+    static constexpr int mids_bytes = 512*4, near_bytes = 2*(1 + 2*TY)*4 + TY*4;
     // front stages: as many as fit, up to three. The copies of a plane take about 2.5 us from issue to
     // completion under load, longer than a plane's work: with two stages the copies' latency set
     // the pace (FP32 256x128x192 without collisions and stores 184 us per step, with them 207)
-    static constexpr int room = 227*1024 - ybuf_bytes - sums_bytes - 1536;
+    static constexpr int room = 227*1024 - ybuf_bytes - sums_bytes - mids_bytes - near_bytes - 1024;
     static constexpr int fit = (room - 2*target_bytes)/front_bytes;
     static constexpr int NFS = fit > 3 ? 3 : fit;
     static constexpr int NTS = NFS*front_bytes + 4*target_bytes <= room ? 4 : 2;
@@ -108,7 +110,8 @@ struct RLay {
     static constexpr int target_off = NFS*front_bytes;
     static constexpr int ybuf_off = target_off + NTS*target_bytes;
     static constexpr int sums_off = ybuf_off + ybuf_bytes;
-    static constexpr int bar_off = sums_off + sums_bytes;
+    static constexpr int mids_off = sums_off + sums_bytes, wz_off = mids_off + mids_bytes, near_off = wz_off + TY*4;
+    static constexpr int bar_off = (wz_off + near_bytes + 7)/8*8;
     // mbarriers: front full, front empty, target full, target empty, ring full and ring free per
     // lane quarter and slot
     static constexpr int B_FF = 0, B_FE = NFS, B_TF = 2*NFS, B_TE = B_TF + NTS, B_RF = B_TE + NTS, B_RE = B_RF + 4*SLOTS;
@@ -473,8 +476,7 @@ struct RoleKernel {
     }
     // Sums of the opposite populations for wall distances below one half, in the order of the paired and
     // gather kernels (x innermost, then y, then xi): FP16 storage carries a changed last place on, and
-    // 2,000 steps over the steep hill (alpha 0.73, whose first rows are such) made 9e-4 of it. (A
-    // twelve-solve burst on 64x32x48: 187 ms, with the sums in y and xi first, x last, 175.)
+    // 2,000 steps over the steep hill (alpha 0.73, whose first rows are such) made 9e-4 of it.
     // y and xi only (populations without an x axis):
     __device__ __forceinline__ V2 bfl_y_xi(int q, int yset, int zset, int x0, int y, int r, int iy) const {
         const size_t N = (size_t)NX*k.NY*k.NZ;
@@ -488,30 +490,35 @@ struct RoleKernel {
         }
         return g;
     }
-    // x, y and xi: a node pair's stencils are five aligned pairs of every row
-    __device__ __forceinline__ V2 bfl_x_y_xi(int q, int xset, int yset, int zset, int x0, int y, int r, int iy) const {
-        const size_t N = (size_t)NX*k.NY*k.NZ;
-        V2 wx[7], g = V2(0.f);
+    // x and y at plane c: a node pair's stencils are five aligned pairs of every row (all loads first: they are one
+    // latency)
+    __device__ __forceinline__ V2 bfl_x_y(int q, int c, int xset, int yset, int x0, int y, int r, int iy) const {
+        const S *plane = fo + q*((size_t)NX*k.NY*k.NZ);
+        V2 f[7][5], wx[7], mid = V2(0.f);
+        float wy[7];
+        int x[5];
 #pragma unroll
-        for (int a = 0; a < 7; a++)   // reference: X weights at [i]
-            wx[a] = k.bfl_mode ? V2(bw(xset, a, r)) : V2(bw(xset, a, x0 + 3), bw(xset, a, x0 + 4));
-#pragma unroll 1
-        for (int c = 0; c < 7; c++) {
-            V2 mid = V2(0.f);
+        for (int m = 0; m < 5; m++) x[m] = (x0 - 4 + 2*m) & (NX - 1);
 #pragma unroll
-            for (int b = 0; b < 7; b++) {
-                const S *p = fo + q*N + bfl_row(c, y - 3 + b);
-                V2 f[5], in = V2(0.f);
+        for (int b = 0; b < 7; b++) {
+            const S *p = plane + (unsigned)bfl_row(c, y - 3 + b);
 #pragma unroll
-                for (int m = 0; m < 5; m++) f[m] = ld2g<S>(p + ((x0 - 4 + 2*m) & (NX - 1)), q);
-#pragma unroll
-                for (int a = 0; a < 7; a++)
-                    in = wx[a]*((a & 1) ? f[(a + 1)/2] : V2(f[a/2].v.y, f[a/2 + 1].v.x)) + in;
-                mid = V2(bw(yset, b, iy))*in + mid;
-            }
-            g = V2(bw(zset, c, r))*mid + g;
+            for (int m = 0; m < 5; m++) f[b][m] = ld2g<S>(p + x[m], q);
         }
-        return g;
+#pragma unroll
+        for (int a = 0; a < 7; a++) {   // reference: X weights at [i], Y weights at [j]
+            wx[a] = V2(bw(xset, a, k.bfl_mode ? r : x0 + 3), bw(xset, a, k.bfl_mode ? r : x0 + 4));
+            wy[a] = bw(yset, a, iy);
+        }
+#pragma unroll
+        for (int b = 0; b < 7; b++) {
+            V2 in = V2(0.f);
+#pragma unroll
+            for (int a = 0; a < 7; a++)
+                in = wx[a]*((a & 1) ? f[b][(a + 1)/2] : V2(f[b][a/2].v.y, f[b][a/2 + 1].v.x)) + in;
+            mid = V2(wy[b])*in + mid;
+        }
+        return mid;
     }
     __device__ __forceinline__ size_t bfl_row(int c, int yy) const {
         const int NY = k.NY;
@@ -521,12 +528,13 @@ struct RoleKernel {
 
     // One flag type of the BFL rows (C/evolution.h:505-572) of a whole row y at plane z <= 1. dst / src:
     // populations set and their opposites, the first without and the other two with an x filter (N3 = 1
-    // or 3). Returns whether the row is set, with the populations (full values) in out.
+    // or 3). Returns 0 where the row is not set, 1 with the populations (full values) in out, 2 where the row is
+    // near: those with an x filter are left to near_rows.
     template <int N3>
-    __device__ __forceinline__ bool bfl_type(V2 *out, int fl, const int (&dst)[N3], const int (&src)[N3], const int (&xset)[N3],
-                                             int yset, int zset, int x0, int y, int z) const {
+    __device__ __forceinline__ int bfl_type(V2 *out, int fl, const int (&dst)[N3], const int (&src)[N3], int yset, int zset, int x0,
+                                            int y, int z) const {
         const int NY = k.NY, nb = 2*k.NYD6, r = z*k.NYD6 + y + 3;
-        if (T.bfl_flag[fl*nb + r] != 1) return false;
+        if (T.bfl_flag[fl*nb + r] != 1) return 0;
         const size_t N = (size_t)NX*NY*k.NZ;
         const float q = T.bfl_q[fl*nb + r];
         if (q > 0.5f) {   // (1/(2Q)) f_opposite + ((2Q-1)/(2Q)) f at the node
@@ -538,11 +546,9 @@ struct RoleKernel {
         if (q < 0.5f) {
             const int iy = k.bfl_mode ? r : y + 3;   // reference: Y weights at [j]
             out[0] = bfl_y_xi(src[0], yset, zset, x0, y, r, iy);
-            if constexpr (N3 == 3)
-#pragma unroll 1
-                for (int m = 1; m < 3; m++) out[m] = bfl_x_y_xi(m == 1 ? src[1] : src[2], m == 1 ? xset[1] : xset[2], yset, zset, x0, y, r, iy);
+            return 2;
         }
-        return q > 0.5f || q < 0.5f;
+        return q > 0.5f ? 1 : 0;
     }
 
     // What the lower wall sets at planes z = 0 and 1 of a node pair: bounce-back (z = 0) and BFL rows. It
@@ -554,9 +560,11 @@ struct RoleKernel {
         V2 bounce[5];      // 5, 11, 12, 15, 16 at z = 0
         unsigned set[2];   // BFL types set at plane z
     };
-    __device__ __forceinline__ void prepare_wall(Wall &w, int z0, int z1, int x0, int y) const {
+    // Called by all collide threads; own: the thread's row is this tile's
+    __device__ __forceinline__ void prepare_wall(unsigned char *smem, Wall &w, int z0, int z1, int x0, int row, int y0, bool own) const {
         const size_t N = (size_t)NX*k.NY*k.NZ;
-        if (z0 == 0) {
+        const int y = y0 + row;
+        if (z0 == 0 && own) {
             const S *b = fo + ((size_t)y*NX + x0);
             w.bounce[0] = ld2g<S>(b + 6*N, 6);
             w.bounce[1] = ld2g<S>(b + 14*N, 14);
@@ -567,12 +575,86 @@ struct RoleKernel {
 #pragma unroll 1
         for (int z = z0; z < z1; z++) {
             V2 *v = w.v[z];
-            unsigned m = bfl_type<3>(v, 0, {3, 7, 8}, {4, 10, 9}, {0, B_XB37, B_XB38}, B_YB378, B_XIB378, x0, y, z) ? 1u : 0u;
-            m |= bfl_type<3>(v + 3, 1, {4, 9, 10}, {3, 8, 7}, {0, B_XB49, B_XB410}, B_YB4910, B_XIB4910, x0, y, z) ? 2u : 0u;
-            m |= bfl_type<1>(v + 6, 2, {15}, {18}, {0}, B_YB15, B_XIB15, x0, y, z) ? 4u : 0u;
-            m |= bfl_type<1>(v + 7, 3, {16}, {17}, {0}, B_YB16, B_XIB16, x0, y, z) ? 8u : 0u;
-            w.set[z] = m;
+            int t[4] = {0, 0, 0, 0};
+            if (own) {
+                t[0] = bfl_type<3>(v, 0, {3, 7, 8}, {4, 10, 9}, B_YB378, B_XIB378, x0, y, z);
+                t[1] = bfl_type<3>(v + 3, 1, {4, 9, 10}, {3, 8, 7}, B_YB4910, B_XIB4910, x0, y, z);
+                t[2] = bfl_type<1>(v + 6, 2, {15}, {18}, B_YB15, B_XIB15, x0, y, z);
+                t[3] = bfl_type<1>(v + 7, 3, {16}, {17}, B_YB16, B_XIB16, x0, y, z);
+            }
+            w.set[z] = (t[0] ? 1u : 0u) | (t[1] ? 2u : 0u) | (t[2] ? 4u : 0u) | (t[3] ? 8u : 0u);
+            if constexpr (TY >= 8) near_rows(smem, v, z, x0, row, y0, t[0] == 2, t[1] == 2);
+            else near_row(v, z, x0, y, t[0] == 2, t[1] == 2);
         }
+    }
+
+    // The populations with an x axis of the thread's row at plane z, where the row is near: 7, 8 (near0: type 0) and 9,
+    // 10 (near1: type 1) into v[1], v[2] and v[4], v[5]. A (row, type) takes 14 sums of 7 x 7 terms, one per
+    // population and plane, each about 1 us of load latency. One after the other, by the row's threads.
+    __device__ __forceinline__ void near_row(V2 *v, int z, int x0, int y, bool near0, bool near1) const {
+        const int r = z*k.NYD6 + y + 3, iy = k.bfl_mode ? r : y + 3;   // reference: Y weights at [j]
+#pragma unroll 1
+        for (int i = 0; i < 4; i++) {
+            const int type = i >> 1, m = i & 1;
+            if (!(type ? near1 : near0)) continue;
+            V2 g = V2(0.f);
+#pragma unroll 1
+            for (int c = 0; c < 7; c++)
+                g = V2(bw(type ? B_XIB4910 : B_XIB378, c, r))*bfl_x_y((type ? 8 : 10) - m, c, (type ? B_XB49 : B_XB37) + m,
+                                                                      type ? B_YB4910 : B_YB378, x0, y, r, iy) + g;
+            v[3*type + 1 + m] = g;
+        }
+    }
+    // The same for tiles of eight or sixteen rows: every row's threads take one sum of any near row at a time, exchanged
+    // through shared memory, and a near row's own threads add its planes in their order. Per step of one
+    // solve on the steep hill (alpha 0.73), against near_row: 64x32x48 FP32 28.9 us (34.1), FP16 29.8 (38.3);
+    // 128x64x96 61.0 (66.7) and 55.5 (60.3); a burst of twelve on 64x32x48 170 ms (185). Tiles of four
+    // rows, as many of them near: 256x128x192 220 us (206).
+    __device__ __forceinline__ void near_rows(unsigned char *smem, V2 *v, int z, int x0, int row, int y0, bool near0, bool near1) const {
+        volatile int *list = (volatile int *)(smem + LY::near_off) + z*(1 + 2*TY);   // number of entries, 2*row + type
+        V2 *mids = (V2 *)(smem + LY::mids_off);                                      // [TY][PR]
+        float *wz = (float *)(smem + LY::wz_off);                                    // [TY], the xi weight of each sum
+        const int j = x0/2;
+        if (j == 0 && near0) list[1 + atomicAdd((int *)list, 1)] = 2*row;
+        if (j == 0 && near1) list[1 + atomicAdd((int *)list, 1)] = 2*row + 1;
+        __syncwarp();
+        bar_sync(BAR_COLLIDE, COLLIDE_THREADS);
+        const int entries = list[0];
+        if (entries == 0) {
+            bar_sync(BAR_COLLIDE, COLLIDE_THREADS);   // every thread has read it before the next wall piece adds to it
+            return;
+        }
+        int at[2] = {0, 0};
+        for (int i = 0; i < entries; i++) {
+            if (list[1 + i] == 2*row) at[0] = 14*i;
+            if (list[1 + i] == 2*row + 1) at[1] = 14*i;
+        }
+        V2 g[2][2] = {{V2(0.f), V2(0.f)}, {V2(0.f), V2(0.f)}};
+#pragma unroll 1
+        for (int base = 0; base < 14*entries; base += TY) {
+            if (base + row < 14*entries) {
+                const int e = list[1 + (base + row)/14], s = (base + row) % 14, m = s >= 7 ? 1 : 0, type = e & 1, ye = y0 + (e >> 1);
+                const int r = z*k.NYD6 + ye + 3, iy = k.bfl_mode ? r : ye + 3;   // reference: Y weights at [j]
+                if (j == 0) wz[row] = bw(type ? B_XIB4910 : B_XIB378, s - 7*m, r);
+                mids[row*PR + j] = bfl_x_y((type ? 8 : 10) - m, s - 7*m, (type ? B_XB49 : B_XB37) + m, type ? B_YB4910 : B_YB378, x0, ye, r, iy);
+            }
+            __syncwarp();
+            bar_sync(BAR_COLLIDE, COLLIDE_THREADS);
+#pragma unroll
+            for (int type = 0; type < 2; type++)
+                if (type ? near1 : near0)
+#pragma unroll
+                    for (int m = 0; m < 2; m++) {
+                        const int first = at[type] + 7*m;
+                        for (int s = max(base, first); s < min(base + TY, first + 7); s++)
+                            g[type][m] = V2(wz[s - base])*mids[(s - base)*PR + j] + g[type][m];
+                    }
+            if (base + TY >= 14*entries && row == 0 && j == 0) list[0] = 0;   // for the next wall piece
+            __syncwarp();
+            bar_sync(BAR_COLLIDE, COLLIDE_THREADS);
+        }
+        if (near0) { v[1] = g[0][0]; v[2] = g[0][1]; }
+        if (near1) { v[4] = g[1][0]; v[5] = g[1][1]; }
     }
 
     // Walls, BFL rows, collision and stores of the node pair (x0, x0 + 1) at row y, plane z, whose
@@ -693,7 +775,7 @@ struct RoleKernel {
         L.own = L.row >= P.yskip;
         if (P.ta <= 1) {
             Wall wall;
-            if (L.own) prepare_wall(wall, P.ta, min(P.tb, 2), L.x0, L.y);
+            prepare_wall(smem, wall, P.ta, min(P.tb, 2), L.x0, L.row, P.y0, L.own);
             collide_targets<true>(smem, P, P.ta, min(P.tb, 2), L, lane, sc, ub, mass, faulted, &wall);
         }
 #pragma unroll 1
@@ -725,6 +807,7 @@ struct RoleKernel {
                 for (int i = 0; i < LY::NTS; i++) { mbar_init(b + LY::B_TF + i, 1); mbar_init(b + LY::B_TE + i, COLLIDE_WARPS); }
                 for (int i = 0; i < 4*SLOTS; i++) { mbar_init(b + LY::B_RF + i, 2); mbar_init(b + LY::B_RE + i, 2); }
                 *(volatile int *)(smem + LY::flag_off) = 0;
+                for (int z = 0; z < 2; z++) ((volatile int *)(smem + LY::near_off))[z*(1 + 2*TY)] = 0;
                 fence_mbar_init();
             }
             __syncwarp();
